@@ -313,6 +313,24 @@ def test_linear_row_does_not_depend_on_batch():
         assert torch.equal(one[0], full[r])
 
 
+@pytest.mark.parametrize("N,K", [(1, 4), (63, 36), (130, 1056), (1024, 3072), (4096, 1028), (2500, 100)])
+@pytest.mark.parametrize("Ms", [(1, 4), (5, 8), (9, 16), (17, 32, 33), (48, 49, 64), (65, 141, 257)])
+def test_float32_linear_at_the_edges_of_its_tiles(Ms, N, K):
+    """The 32-bit product at the edges of its row tiles, of 64 weight rows, of k-blocks of 32 and of the shares of K (1 056
+    in eight shares of 160: the last has none) against 64 bits.  A sum of K terms in float32, in whatever order, is off by at
+    most (K + 8) 2^-24 sum |x w|; a row's bits are the same whatever the number of rows."""
+    w = _randn((N, K), torch.float32, 9).to(DEV)
+    x = _randn((max(Ms), K), torch.float32, 8).to(DEV)
+    one = torch.empty(1, N, device=DEV)
+    ops.linear(x[:1].contiguous(), w, one)
+    for M in Ms:
+        got = torch.full((M + 1, N), 7.0, device=DEV)
+        ops.linear(x[:M].contiguous(), w, got[:M])
+        err = (got[:M].double() - x[:M].double() @ w.double().T).abs()
+        assert (err <= (K + 8) * 2.0 ** -24 * (x[:M].double().abs() @ w.double().abs().T)).all()
+        assert torch.equal(got[0], one[0]) and (got[M] == 7.0).all()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,I", [(1, 10), (9, 224), (33, 1001)])
 def test_silu_mul(dtype, T, I):
