@@ -1,28 +1,34 @@
 // The float32 product (see gemm_f32.cuh): every multiply-add is a float32 fma, two at a time (`fma.rn.f32x2`).
 //
-// Order of a sum, whatever M is: K is cut into S equal chunks (a function of N and K alone), a chunk is summed as two
-// chains, one over its even and one over its odd k, the chunk's sum is even + odd, and the chunks are added in order.  So a
-// row's bits do not depend on what else is in the batch, and the chains are 2 S times shorter than one over all of K.
+// Order of a sum, whatever M is: K is cut into S equal chunks (a function of N and K alone), a chunk into runs of 16 that
+// are dealt to four groups in turn; a group's k are summed as two chains, the even and the odd ones, and even + odd, the
+// groups and the chunks are added in order.  So a row's bits do not depend on
+// what else is in the batch, and the chains are 8 S times shorter than one over all of K.
 //
 // What bounds it: a few rows stream the weights, 4 bytes for each, and some hundreds of rows are bound by the float32
 // multiply-adds.  Hence
-//  - both operands go into shared memory as they lie (k fastest, rows padded to 36 floats: eight rows' 16-byte words are
-//    conflict-free) by 16-byte cp.async, several k-blocks of 32 ahead; with at most 16 rows the weights' first blocks are
+//  - both operands go into shared memory as they lie (k fastest, rows padded by four floats: eight rows' 16-byte words
+//    are conflict-free) by 16-byte cp.async, several k-blocks ahead; with at most 16 rows the weights' first blocks are
 //    asked for before the wait for the kernel before;
 //  - a thread keeps TM x TN pairs of sums and reads 4 k of a row in one load: the pair (k, k + 1) is the register pair that
-//    the two-wide fma takes, so nothing is packed or duplicated;
+//    the two-wide fma takes, so nothing is packed or duplicated; up to 8 x 8 sums, since a 16-byte load from shared memory
+//    costs four of its cycles even where lanes read the same word;
+//  - up to 16 rows the four groups are warps of their own, so that a tile has enough of them to hide its loads (a block is 64
+//    k, a run of each); beyond, a thread takes one group after the other (a block is two runs of a group);
 //  - tiles are 64 weight rows, and a cluster of S CTAs shares K where the tiles alone would leave SMs idle; the partial
 //    tiles meet through distributed shared memory, each CTA finishing a share of the outputs;
 //  - the tile's height is the smallest of 4, 8, 16 that takes all rows, beyond that the one of 32, 48, 64 that wastes least.
-// Measured on a B200, chains of launches over weights larger than L2: 4096 x 1024 at 3 rows 7.3 us (2.3 TB/s), 151936 x 1024 at
-// 3 rows 186 us (3.3 TB/s), 6144 x 1024 at 141 rows 52 us (34 TFLOP/s).  Qwen3-0.6B in float32, 141 prompt tokens and four
-// steps of three tokens: 164 ms with the kernel of gemm_generic.cu (scalar loads, a CTA's one chain over all of K), of which
-// the products were 93 %; 17.8 ms with this one.
+// Measured on a B200, chains of launches over weights larger than L2: 4096 x 1024 at 3 rows 5.5 us (3.1 TB/s), 151936 x 1024
+// at 3 rows 99 us (6.3 TB/s), 6144 x 1024 at 141 rows 57 us (31 TFLOP/s).  With two threads' worth of k in one group and
+// four rows of one column a thread, 3 rows took 7.3 and 186 us; 8 x 8 sums a thread from 32 rows on (8 warps an SM instead
+// of 12) took 74 us at 141 rows.  Qwen3-0.6B in float32, 141 prompt tokens and four steps of three tokens: 164 ms with
+// the kernel of gemm_generic.cu (scalar loads, a CTA's one chain over all of K), of which the products were 93 %; 11.9 ms
+// with this one and the attention kernel of attention_generic.cu as it is now (5.1 of those 164 ms were saved there).
 #include "gemm_f32.cuh"
 
 #define GF_BN 64
-#define GF_BK 32
-#define GF_LD (GF_BK + 4)
+#define GF_GROUPS 4
+#define GF_RUN 16                     // consecutive k of a group
 
 __device__ __forceinline__ void gf_copy16(float* smem, const float* gmem, bool valid) {
   const int bytes = valid ? 16 : 0;                     // nothing is read for a place outside; the 16 bytes become zeros
@@ -35,43 +41,57 @@ __device__ __forceinline__ void gf_fma2(unsigned long long& acc, unsigned long l
 
 template <int BM, int TM, int TN, int STAGES>
 struct GfShape {
-  static constexpr int MT = BM / TM, NT = GF_BN / TN, THREADS = MT * NT;
+  static constexpr bool SLICED = BM <= 16;                                      // the groups are warps of their own
+  static constexpr int MT = BM / TM, NT = GF_BN / TN, GROUP = MT * NT, THREADS = SLICED ? GF_GROUPS * GROUP : GROUP;
   static constexpr int LANES_M = MT >= 4 ? 4 : MT, LANES_N = 32 / LANES_M;      // a warp's threads over the tile
-  static constexpr int STAGE = (GF_BN + BM) * GF_LD;                            // floats
+  static constexpr int CTAS = BM == 64 ? 2 : 3;                                 // an SM's registers hold at least
+  static constexpr int BK = SLICED ? GF_GROUPS * GF_RUN : 2 * GF_RUN;           // k of a loaded block
+  static constexpr int LD = BK + 4;
+  static constexpr int STAGE = (GF_BN + BM) * LD;                            // floats
   static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(float);
-  static_assert(THREADS % 32 == 0 && NT % LANES_N == 0 && MT % LANES_M == 0, "whole warps");
-  static_assert((size_t)BM * GF_BN * sizeof(float) <= SMEM, "the partial tile takes the stages' place");
+  static_assert(GROUP % 32 == 0 && NT % LANES_N == 0 && MT % LANES_M == 0, "whole warps");
+  static_assert((size_t)(SLICED ? GF_GROUPS : 1) * BM * GF_BN * sizeof(float) <= SMEM, "the groups' partial tiles take the stages' place");
 };
 
 template <int BM, int TM, int TN, int STAGES>
-__global__ void __launch_bounds__(GfShape<BM, TM, TN, STAGES>::THREADS)
+__global__ void __launch_bounds__(GfShape<BM, TM, TN, STAGES>::THREADS, GfShape<BM, TM, TN, STAGES>::CTAS)
 gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out,
                 int M, int N, int K, int chunk, int splits, int act, int vec) {
   using S = GfShape<BM, TM, TN, STAGES>;
-  constexpr bool EARLY = BM <= 16;
+  constexpr bool EARLY = S::SLICED;
   extern __shared__ __align__(16) float gf_smem[];
   const int rank = blockIdx.x % splits;
   const int n0 = blockIdx.x / splits * GF_BN, m0 = blockIdx.y * BM;
   const int k_begin = min(K, rank * chunk), k_end = min(K, k_begin + chunk);
-  const int blocks = (k_end - k_begin + GF_BK - 1) / GF_BK;
-  constexpr int WORDS = GF_BK / 4;                      // 16-byte words of a row's k-block
-
+  // blocks to load: of a run of each group; or, where a thread takes the groups in turn, `turn` of two runs for each
+  const int rounds = (k_end - k_begin + GF_GROUPS * GF_RUN - 1) / (GF_GROUPS * GF_RUN);
+  const int turn = (rounds + 1) / 2;
+  const int blocks = S::SLICED ? rounds : turn * GF_GROUPS;
+  constexpr int LD = S::LD, WORDS = S::BK / 4;                      // 16-byte words of a row's k-block
+  static_assert(S::THREADS % WORDS == 0, "a thread's words are the same one of every row");
+  const int word = threadIdx.x % WORDS, row = threadIdx.x / WORDS;
+  const int word_k = S::SLICED ? word * 4 : word / (GF_RUN / 4) * (GF_GROUPS * GF_RUN) + word % (GF_RUN / 4) * 4;
+  auto k_of = [&](int b) {                              // the k of this thread's word of block b
+    if (S::SLICED) return k_begin + b * S::BK + word_k;
+    const int group = b / turn;
+    return k_begin + (b - group * turn) * (2 * GF_GROUPS * GF_RUN) + group * GF_RUN + word_k;
+  };
   auto load_w = [&](int b) {
-    float* ws = gf_smem + (b % STAGES) * S::STAGE;
+    float* ws = gf_smem + (b % STAGES) * S::STAGE + word * 4;
+    const int k = k_of(b);
 #pragma unroll
-    for (int e = threadIdx.x; e < GF_BN * WORDS; e += S::THREADS) {
-      const int r = e / WORDS, k = k_begin + b * GF_BK + (e % WORDS) * 4;
+    for (int r = row; r < GF_BN; r += S::THREADS / WORDS) {
       const bool ok = n0 + r < N && k < k_end;
-      gf_copy16(ws + r * GF_LD + (e % WORDS) * 4, ok ? w + (size_t)(n0 + r) * K + k : w, ok);
+      gf_copy16(ws + r * LD, ok ? w + (size_t)(n0 + r) * K + k : w, ok);
     }
   };
   auto load_x = [&](int b) {
-    float* xs = gf_smem + (b % STAGES) * S::STAGE + GF_BN * GF_LD;
+    float* xs = gf_smem + (b % STAGES) * S::STAGE + GF_BN * LD + word * 4;
+    const int k = k_of(b);
 #pragma unroll
-    for (int e = threadIdx.x; e < BM * WORDS; e += S::THREADS) {
-      const int r = e / WORDS, k = k_begin + b * GF_BK + (e % WORDS) * 4;
+    for (int r = row; r < BM; r += S::THREADS / WORDS) {
       const bool ok = m0 + r < M && k < k_end;
-      gf_copy16(xs + r * GF_LD + (e % WORDS) * 4, ok ? x + (size_t)(m0 + r) * K + k : x, ok);
+      gf_copy16(xs + r * LD, ok ? x + (size_t)(m0 + r) * K + k : x, ok);
     }
   };
 
@@ -90,7 +110,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
 
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, group = threadIdx.x / S::GROUP, warp = threadIdx.x % S::GROUP >> 5;
   const int tm = lane % S::LANES_M + S::LANES_M * (warp % (S::MT / S::LANES_M));
   const int tn = lane / S::LANES_M + S::LANES_N * (warp / (S::MT / S::LANES_M));
   unsigned long long acc[TM][TN];                       // (sum over even k, sum over odd k)
@@ -98,22 +118,28 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+  float total[TM][TN];                                  // the groups before
+  auto even_and_odd = [&](int i, int j) {
+    return __uint_as_float((unsigned)(acc[i][j] & 0xffffffffull)) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+  };
 
+  const int offset = S::SLICED ? group * GF_RUN : 0;
+  int left = turn;                                      // blocks of the group in turn
 #pragma unroll 1
   for (int b = 0; b < blocks; ++b) {
     asm volatile("cp.async.wait_group %0;\n" :: "n"(STAGES - 2) : "memory");
     __syncthreads();                                    // block b has landed; block b - 1 is read no more
     if (b + STAGES - 1 < blocks) { load_w(b + STAGES - 1); load_x(b + STAGES - 1); }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const float* ws = gf_smem + (b % STAGES) * S::STAGE + tn * GF_LD;
-    const float* xs = gf_smem + (b % STAGES) * S::STAGE + (GF_BN + tm) * GF_LD;
+    const float* ws = gf_smem + (b % STAGES) * S::STAGE + tn * LD + offset;
+    const float* xs = gf_smem + (b % STAGES) * S::STAGE + (GF_BN + tm) * LD + offset;
 #pragma unroll
-    for (int k = 0; k < GF_BK; k += 4) {
+    for (int k = 0; k < (S::SLICED ? GF_RUN : S::BK); k += 4) {
       ulonglong2 a[TM], c[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * S::MT * GF_LD + k);
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * S::MT * LD + k);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) c[j] = *reinterpret_cast<const ulonglong2*>(ws + j * S::NT * GF_LD + k);
+      for (int j = 0; j < TN; ++j) c[j] = *reinterpret_cast<const ulonglong2*>(ws + j * S::NT * LD + k);
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -123,17 +149,38 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
 #pragma unroll
         for (int j = 0; j < TN; ++j) gf_fma2(acc[i][j], a[i].y, c[j].y);
     }
+    if (!S::SLICED && --left == 0) {
+      left = turn;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          total[i][j] = b < turn ? even_and_odd(i, j) : total[i][j] + even_and_odd(i, j);
+          acc[i][j] = 0ull;
+        }
+    }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  // the CTA's partial tile [BM][64] in the stages' place
+  // the CTA's partial tile [BM][64] in the stages' place (the groups' four, added into the first)
+  constexpr int TILE = BM * GF_BN;
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const float even = __uint_as_float((unsigned)(acc[i][j] & 0xffffffffull)), odd = __uint_as_float((unsigned)(acc[i][j] >> 32));
-      gf_smem[(tm + i * S::MT) * GF_BN + tn + j * S::NT] = even + odd;
+    for (int j = 0; j < TN; ++j)
+      gf_smem[(S::SLICED ? group * TILE : 0) + (tm + i * S::MT) * GF_BN + tn + j * S::NT] = S::SLICED || blocks == 0 ? even_and_odd(i, j) : total[i][j];
+  if (S::SLICED) {
+    __syncthreads();
+    for (int e = threadIdx.x * 4; e < TILE; e += S::THREADS * 4) {
+      float4 v = *reinterpret_cast<const float4*>(gf_smem + e);
+#pragma unroll
+      for (int g = 1; g < GF_GROUPS; ++g) {
+        const float4 p = *reinterpret_cast<const float4*>(gf_smem + g * TILE + e);
+        v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+      }
+      *reinterpret_cast<float4*>(gf_smem + e) = v;
     }
+  }
   if (splits > 1) cluster_sync_all(); else __syncthreads();
   for (int e = (rank * S::THREADS + threadIdx.x) * 4; e < BM * GF_BN; e += splits * S::THREADS * 4) {
     const int gm = m0 + e / GF_BN, gn = n0 + e % GF_BN;
@@ -183,10 +230,10 @@ int qe_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K,
   const int tiles = (N + GF_BN - 1) / GF_BN;
   int splits = 1;
   while (splits < 8 && (long)tiles * splits * 2 <= 2 * 148 && K / (2 * splits) >= 128) splits *= 2;
-  const int chunk = ((K + splits - 1) / splits + GF_BK - 1) / GF_BK * GF_BK;
-  if (M <= 4) return gf_launch<4, 4, 1, 8>(x, w, out, M, N, K, chunk, splits, act, stream);
-  if (M <= 8) return gf_launch<8, 4, 1, 8>(x, w, out, M, N, K, chunk, splits, act, stream);
-  if (M <= 16) return gf_launch<16, 4, 2, 6>(x, w, out, M, N, K, chunk, splits, act, stream);
+  const int chunk = ((K + splits - 1) / splits + GF_GROUPS * GF_RUN - 1) / (GF_GROUPS * GF_RUN) * (GF_GROUPS * GF_RUN);
+  if (M <= 4) return gf_launch<4, 4, 2, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
+  if (M <= 8) return gf_launch<8, 8, 2, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
+  if (M <= 16) return gf_launch<16, 8, 4, 3>(x, w, out, M, N, K, chunk, splits, act, stream);
   // rows that the tiles cover, a tile's own cost counted as 8 more
   auto cost = [&](long bm) { return (M + bm - 1) / bm * (bm + 8); };
   if (M > 4096 || (cost(64) <= cost(48) && cost(64) <= cost(32))) return gf_launch<64, 8, 4, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
