@@ -398,17 +398,38 @@ decode_attention_mma_kernel(FaArgs A_launch, long long prefetch_delta, int early
       __threadfence();
       for (int e = tid; e < nrows * D; e += DM_THREADS) {
         const int r = e / D, d = e - r * D;
-        float m = -INFINITY;
-        for (int sp = 0; sp < n_splits; ++sp)
-          m = fmaxf(m, __ldcg(A.part_ml + 2 * ((((size_t)first + sp) * Hkv + hkv) * A.part_rows + r)));
-        const float mb = m == -INFINITY ? 0.f : m;
-        float l = 0.f, acc = 0.f;
-        for (int sp = 0; sp < n_splits; ++sp) {
-          const size_t slot = (((size_t)first + sp) * Hkv + hkv) * A.part_rows + r;
-          const float wgt = exp2f(__ldcg(A.part_ml + 2 * slot) - mb);
-          l += wgt * __ldcg(A.part_ml + 2 * slot + 1);
-          acc += wgt * __ldcg(A.part_acc + slot * D + d);
+        // eight parts at a time, all of their loads on their way together (a part after the other was a chain of L2 round
+        // trips, two for each part, behind the step's last keys)
+        float m = -INFINITY, l = 0.f, acc = 0.f;
+        for (int sp0 = 0; sp0 < n_splits; sp0 += 8) {
+          float2 ml[8];
+          float aa[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            ml[i] = make_float2(-INFINITY, 0.f);
+            aa[i] = 0.f;
+            if (sp0 + i < n_splits) {
+              const size_t slot = (((size_t)first + sp0 + i) * Hkv + hkv) * A.part_rows + r;
+              ml[i] = __ldcg(reinterpret_cast<const float2*>(A.part_ml) + slot);
+              aa[i] = __ldcg(A.part_acc + slot * D + d);
+            }
+          }
+          float m_new = m;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) m_new = fmaxf(m_new, ml[i].x);
+          const float base = m_new == -INFINITY ? 0.f : m_new;
+          const float keep = exp2f(m - base);
+          l *= keep;
+          acc *= keep;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float wgt = exp2f(ml[i].x - base);
+            l += wgt * ml[i].y;
+            acc += wgt * aa[i];
+          }
+          m = m_new;
         }
+        const float mb = m == -INFINITY ? 0.f : m;
         const int ti = r / G, hg = r - ti * G;
         if (A.sinks) l += exp2f(A.sinks[hkv * G + hg] * 1.4426950408889634f - mb);    // the sink's share of the denominator
         out_row0[(size_t)ti * ((size_t)Hq * out_hd) + (size_t)(hkv * G + hg) * out_hd + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);

@@ -242,9 +242,11 @@ class ModelRunner:
         if self.use_cuda_graphs and all(n == 1 for n in q_lens):
             buckets = tuple(-(-max(len(e.cache.tables[g.index]) for e in entries) // B) * B
                             for g in cache.paged_groups)
-            graph_key = (R, N, buckets)
             uniform_splits = ops.decode_splits(R, max(buckets, default=B) * cache.page_size,
-                                               self.model.attention_geometries, self.dtype)
+                                               self.model.attention_geometries, self.dtype, ctx_lens)
+            # contexts of unequal lengths may be cut by their lengths: other launches, a graph of their own
+            by_length = tuple(type(p) is ops.TotalParts for p in uniform_splits.values())
+            graph_key = (R, N, buckets + by_length if any(by_length) else buckets)
         elif self.use_cuda_graphs and self.capture_all_steps:
             # block tables padded to 64 x a power of two entries, so that few widths occur
             buckets = tuple(B << max(0, (-(-max(len(e.cache.tables[g.index]) for e in entries) // B) - 1).bit_length())

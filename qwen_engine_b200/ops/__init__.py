@@ -9,6 +9,7 @@ operation lives with the tests (tests/ref_ops.py).
 from __future__ import annotations
 
 import ctypes
+import heapq
 import os
 import struct
 from typing import Optional
@@ -51,6 +52,9 @@ DECODE_ATTENTION_MMA_EARLY = True   # that kernel requests earlier steps' keys b
 DECODE_ATTENTION_MMA_BESIDE_TC = True   # also for the decoded tokens of a step whose prompt portions go to the tcgen05 kernel
 SHIFTS_IN_ONE_LAUNCH = True          # a mixer that mixes its heads' weights: the shifts of the values' kv head as one launch where the step has no long portion
 DECODE_ATTENTION_MMA_WIDE = True    # steps with at most as many attention CTAs as SMs: CTAs of 8 warps, one per SM (and contexts split for 148 CTAs, not 296)
+DECODE_PARTS_BY_LENGTH = True          # decode steps of many requests with contexts of unequal lengths: parts in proportion to them
+DECODE_PART_MIN_KEYS = 256             # ... none shorter than this
+DECODE_PART_COST_KEYS = 96             # what the merge of a cut context costs, in keys of a CTA of 4 warps
 LATENT_DECODE = True                 # decoded tokens over a latent cache (one plane, one kv head): the kernel whose warps stream key groups of their own
 LATENT_DECODE_MIN_PART = 128         # keys of a part at least where a step's contexts are cut for that kernel
 DECODE_PREFETCH_KV_MB = 12          # that kernel asks L2 for the next layer's keys and values when a layer's are at most this many MB (0: never).  Measured (0.6B, context 1 024, asked for before the kernel's dependency wait): 4.4 MB (one request) 0.698 -> 0.690 ms a step, 8.8 MB 0.777 -> 0.765, 17.6 MB equal, 35 MB (eight) 0.915 -> 0.957
@@ -1014,6 +1018,47 @@ def value_block_size(key_dim: int, value_dim: int) -> tuple[int, int]:
     return up(max(key_dim, value_dim)), 1
 
 
+class TotalParts(int):
+    """In ``uniform_splits``, in the place of a number of parts per request: the work items of all requests together."""
+
+
+def attended_keys(q_len: int, ctx_len: int, window: int) -> int:
+    """The keys that a request's parts are cut from (from the window's first key tile on)."""
+    return ctx_len + q_len - (max(0, ctx_len - window + 1) // FLASH_BN * FLASH_BN if window else 0)
+
+
+def parts_by_length(keys: list[int], total: int) -> list[int]:
+    """How many parts each of the requests with so many keys is cut into, at most ``total`` in all (at least one each): the
+    next part goes to the request whose parts are longest, until those are short."""
+    parts = [1] * len(keys)
+    longest = [(-n, i) for i, n in enumerate(keys)]
+    heapq.heapify(longest)
+    for _ in range(total - len(keys)):
+        n, i = longest[0]
+        if -n < 2 * DECODE_PART_MIN_KEYS and -keys[i] / (parts[i] + 1) > -DECODE_PART_MIN_KEYS:
+            break
+        parts[i] += 1
+        heapq.heapreplace(longest, (-keys[i] / parts[i], i))
+    return parts
+
+
+def parts_for_lengths(geo, keys: list[int], one_each: int) -> Optional[TotalParts]:
+    """The work items to deal out by length among requests with so many keys where that is faster than contexts of which the
+    longest part has ``one_each`` keys (in keys of a CTA of 4 warps, two per SM); None where it is not.
+
+    The longest part sets the time, or the keys of all where the parts are even.  Measured on a B200 (kv heads 8, a chain of
+    launches): 28 requests of 130 to 2 045 keys 37.2 us whole, 27.5 in 37 parts (one wave), 31.8 in 55; 15 such 24.8 whole (8
+    warps each), 16.0 in 37 parts; 64 of 985 on average 56.7 whole, 51.6 in 74 (two waves); one of 16 384 beside 15 of 200
+    199 whole, 22.6 in 37.  Contexts of equal lengths gain nothing (16 of 1 400: 20.9 whole, 22.1 in 37) and stay whole."""
+    slots = FLASH_TARGET_CTAS // (geo[1] * value_blocks(geo))
+    total = slots if len(keys) < slots else 2 * slots
+    if not DECODE_PARTS_BY_LENGTH or slots < 1 or len(keys) >= total or total * geo[1] * value_blocks(geo) > _MERGE_COUNTERS:
+        return None
+    even = sum(keys) / slots
+    longest = max(-(-n // p) for n, p in zip(keys, parts_by_length(keys, total)))
+    return TotalParts(total) if max(longest, even) + DECODE_PART_COST_KEYS < max(one_each, even) else None
+
+
 def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
                    geometries=(), dtype: torch.dtype = torch.float32,
                    uniform_splits: Optional[dict] = None) -> dict[str, list[int]]:
@@ -1027,8 +1072,9 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
     request if all are cut into the same 2, 4 or 8 parts (they can then form clusters) else 0]; requests that bring many rows go to the tcgen05 kernel
     instead where it takes the geometry: ``tc<i>_items``, ``tc<i>_sched`` (which CTA runs which
     item for which kv head) and ``tc<i>_info`` = [parts, rows per part, CTAs].
-    ``uniform_splits`` (geometry -> number of parts) fixes the number of parts of every request,
-    so that the lists depend on the batch's shape only (for steps replayed from a CUDA graph)."""
+    ``uniform_splits`` (geometry -> number of parts) fixes the number of parts of every request, or (``TotalParts``) the
+    number of work items of all of them, which are then dealt out by length, so that the lists' lengths depend on the
+    batch's shape only (for steps replayed from a CUDA graph)."""
     tiles: list[int] = []
     for r, n in enumerate(q_lens):
         for q0 in range(0, n, ATTN_TILE_Q):
@@ -1050,6 +1096,18 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
         merge: list[int] = []
         n_parts, part_rows, row0, max_rows = 0, 1, 0, 0
         whole: list[tuple[int, list[int]]] = []        # (keys the tile visits, its work item)
+        # parts in proportion to the contexts' lengths: as the caller fixed it, or for decoded tokens beside prompt portions
+        items_in_all, shares = None, {}
+        rest = [r for r, tc in enumerate(on_tc) if not tc]
+        if uniform_splits is not None:
+            items_in_all = uniform_splits[geo] if isinstance(uniform_splits[geo], TotalParts) else None
+        elif (rest and len(rest) < len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_BESIDE_TC and D == 128
+              and geometry_planes(geo) >= 2 and max(q_lens[r] for r in rest) * G <= 16):
+            at_most = max(1, FLASH_TARGET_CTAS // base)
+            keys = [attended_keys(q_lens[r], ctx_lens[r], window) for r in rest]
+            items_in_all = parts_for_lengths(geo, keys, max(-(-k // min(-(-k // FLASH_SPLIT), at_most)) for k in keys))
+        if items_in_all is not None:
+            shares = dict(zip(rest, parts_by_length([attended_keys(q_lens[r], ctx_lens[r], window) for r in rest], items_in_all)))
         for r, (n, c) in enumerate(zip(q_lens, ctx_lens)):
             total = c + n
             if on_tc[r]:
@@ -1060,7 +1118,9 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
                     tc_tiles.append((-(-(hi - lo // TC_BN * TC_BN) // TC_BN), lo, hi, (r, q0, row0, n, c)))
                 row0 += n
                 continue
-            if uniform_splits is not None:
+            if shares:
+                splits = shares[r]
+            elif uniform_splits is not None:
                 splits = uniform_splits[geo]
             else:
                 lo = (max(0, c - window + 1) // FLASH_BN) * FLASH_BN if window else 0
@@ -1069,7 +1129,11 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
                     splits = min(-(-(total - lo) // FLASH_SPLIT), max(1, FLASH_TARGET_CTAS // base))
             if splits > 1:
                 for sp in range(splits):
-                    items += [r, 0, 0, 0, n_parts + sp, splits, sp, row0, n, c, 0, 0]
+                    item = [r, 0, 0, 0, n_parts + sp, splits, sp, row0, n, c, 0, 0]
+                    if shares:
+                        whole.append((-(-total // splits), item))
+                    else:
+                        items += item
                 merge += [r, 0, n_parts, splits]
                 n_parts += splits
                 part_rows = max(part_rows, n * G)
@@ -1081,10 +1145,15 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
         # tiles that visit many keys start first, so that the last wave of CTAs is made of short ones
         whole.sort(key=lambda kv: -kv[0])
         items = [x for _, item in whole for x in item] + items
+        if items_in_all is not None:
+            # the lists, the scratch and the launch are those of the total, whatever the lengths: what is left over are items
+            # without rows; the kernel's last part merges, no list of merges is needed
+            items += ([0, 0, 0, 0, -1] + [0] * (FLASH_ITEM_INTS - 5)) * (items_in_all - len(items) // FLASH_ITEM_INTS)
+            n_parts, part_rows, merge = int(items_in_all), max(q_lens[r] for r in rest) * G, []
         plan[f"fa{gi}_items"] = items
         plan[f"fa{gi}_merge"] = merge
         sizes = {m for m in merge[3::4]}
-        same = sizes.pop() if len(sizes) == 1 and not whole else 0
+        same = sizes.pop() if len(sizes) == 1 and not whole and items_in_all is None else 0
         plan[f"fa{gi}_info"] = [n_parts, part_rows, int(max_rows <= 16), max_rows, same if same in (2, 4, 8) else 0]
         if tc_tiles and latent_tc:
             # a tile's keys are not cut: the tiles alone, those with the most keys first
@@ -1102,9 +1171,10 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
 DECODE_CLUSTER4_MAX_SPAN = 4096   # keys up to which 4 parts in a cluster are preferred to more parts merged through memory
 
 
-def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype) -> dict:
+def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype, ctx_lens: Optional[list] = None) -> dict:
     """The fixed number of parts per request for a decode step of ``num_reqs`` requests whose block
-    tables hold up to ``max_tokens`` tokens: enough parts to fill the GPU, none shorter than a split."""
+    tables hold up to ``max_tokens`` tokens: enough parts to fill the GPU, none shorter than a split.
+    With the requests' ``ctx_lens``, contexts that would stay whole may be cut by their lengths instead (``TotalParts``)."""
     out = {}
     for geo in geometries:
         Hq, Hkv, D, window, _ = split_geometry(geo)
@@ -1142,6 +1212,11 @@ def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype
             elif span <= DECODE_CLUSTER4_MAX_SPAN:
                 parts = 4
         out[geo] = parts
+        if (ctx_lens and parts == 1 and DECODE_ATTENTION_MMA and dtype == torch.bfloat16 and D == 128 and Hq // Hkv <= 16
+                and geometry_planes(geo) >= 2):
+            keys = [attended_keys(1, c, window) for c in ctx_lens]
+            wide = DECODE_ATTENTION_MMA_WIDE and num_reqs * Hkv <= TC_TARGET_CTAS          # CTAs of 8 warps
+            out[geo] = parts_for_lengths(geo, keys, -(-max(keys) // (2 if wide else 1))) or parts
     return out
 
 

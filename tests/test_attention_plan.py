@@ -93,3 +93,44 @@ def test_long_tiles_are_cut_only_where_the_schedule_gains():
     assert many["tc0_info"][0] == 0, "enough tiles for every SM: nothing is cut"
     behind = ops.plan_attention([128], [30000], 16, geo, torch.bfloat16)
     assert behind["tc0_info"][0] >= 2, "one tile behind a long context is cut so that more than 8 SMs work"
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_parts_by_length_cover_every_key_in_a_fixed_number_of_items(seed):
+    """Decoded tokens whose contexts are cut by their lengths: the lists' lengths and the scratch depend on the total alone, every
+    request has the parts it was given, longest first, and what is left over are items without rows."""
+    rng = random.Random(200 + seed)
+    geo = ((16, 8, 128, 0), (32, 8, 128, 0), (16, 8, 128, 700, True), (16, 8, 128, 0, False, 3))[seed % 4]
+    R = rng.randint(10, 18)
+    ctx = [rng.choice([0, 1, 200, 255, 256, 3000, 9000, rng.randint(1, 2000)]) for _ in range(R)]
+    total = ops.TotalParts(rng.choice([R, R + 1, 37, 74]))
+    plan = ops.plan_attention([1] * R, ctx, 16, (geo,), torch.bfloat16, uniform_splits={geo: total})
+    items = _items(plan, "fa0_items")
+    assert len(items) == total and plan["fa0_info"] == [total, geo[0] // geo[1], 1, geo[0] // geo[1], 0] and plan["fa0_merge"] == []
+    of = {r: [i for i in items if i[8] and i[0] == r] for r in range(R)}
+    parts = ops.parts_by_length([ops.attended_keys(1, c, geo[3]) for c in ctx], total)
+    used = [i[4] for i in items if i[4] >= 0]
+    assert len(set(used)) == len(used) and max(used, default=0) < total
+    for r, mine in of.items():
+        assert len(mine) == parts[r] and all(i[7] == r and i[9] == ctx[r] for i in mine)
+        if len(mine) == 1:
+            assert mine[0][2:7] == [0, ctx[r] + 1, -1, 0, 0]
+        else:
+            mine.sort(key=lambda i: i[6])
+            assert [i[4:7] for i in mine] == [[mine[0][4] + s, len(mine), s] for s in range(len(mine))]
+    empty = [i for i in items if not i[8]]
+    assert len(empty) == total - sum(parts) and all(i == [0, 0, 0, 0, -1] + [0] * 7 for i in empty)
+
+
+def test_contexts_are_cut_by_length_only_where_they_are_unequal():
+    geo, bf = (16, 8, 128, 0), torch.bfloat16
+    even, ragged = [1000] * 28, [150 + 70 * i for i in range(28)]
+    splits = lambda ctx, dtype=bf, g=geo: ops.decode_splits(len(ctx), 2048, (g,), dtype, ctx)[g]
+    assert type(splits(ragged)) is ops.TotalParts and splits(ragged) == 37
+    assert splits(even) == 1 and type(splits(even)) is int
+    assert splits(ragged[:4]) > 1 and type(splits(ragged[:4])) is int, "few requests are cut into clusters"
+    assert type(splits(ragged, torch.float32)) is int and type(splits(ragged, g=(16, 8, 64, 0))) is int
+    assert type(splits([100 + 10 * i for i in range(28)])) is int, "short contexts stay whole"
+    assert splits(ragged * 2 + ragged[:8]) == 74 and type(splits(ragged * 3)) is int
+    beside = ops.plan_attention([512] + [1] * 15, [0] + [150 + 130 * i for i in range(15)], 16, (geo,), bf)
+    assert len(_items(beside, "fa0_items")) == beside["fa0_info"][0] == 37

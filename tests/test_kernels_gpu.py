@@ -659,6 +659,23 @@ def test_decode_attention_mma_many_rows(Hq, Hkv, P, q_lens, ctx_lens, window, st
     _close(got, want, dtype)
 
 
+@pytest.mark.parametrize("Hq,Hkv,P,window", [(16, 8, 16, 0), (32, 8, 16, 0), (16, 8, 8, 100), (8, 8, 12, 0), (32, 2, 64, 0)])
+@pytest.mark.parametrize("ctx_lens", [[0, 15, 300, 2023, 47, 800, 31, 555, 1200, 16], [3] * 8 + [5000, 7]])
+@pytest.mark.parametrize("total", [10, 13, 37])
+def test_decode_attention_parts_by_length(Hq, Hkv, P, window, ctx_lens, total, decode_kernel):
+    """A decode step whose contexts are cut in proportion to their lengths: whole ones, up to 28 parts of one (merged eight at a
+    time), items without rows; against the plain reference."""
+    D, dtype = 128, torch.bfloat16
+    q_lens = [1] * len(ctx_lens)
+    case = _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed=61)
+    want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ref_ops.paged_attention, "cpu")
+    for _ in range(2):                                  # (the second launch finds the counters as the first left them)
+        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, uniform=ops.TotalParts(total))
+        assert ops.last_attention_kernel == "decode_attention_mma"
+        _close(got, want, dtype)
+    assert int(ops._merge_counters(torch.device(DEV)).abs().max()) == 0
+
+
 def test_decode_attention_mma_asks_for_the_next_layers_cache(monkeypatch):
     """With another layer's cache given (and allowed by size), the kernel asks L2 for that layer's keys and
     values: the output is the same bits, and nothing of the other cache changes."""
