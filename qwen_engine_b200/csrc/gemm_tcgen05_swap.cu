@@ -86,21 +86,21 @@ gemm_tcgen05_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     }
   } else if (warp == 1) {
     // ---- MMA issuer -------------------------------------------------------------------------------
-    if (lane == 0) {
+    {                                                 // (the whole warp: one lane is elected per instruction)
       const uint32_t idesc = make_idesc(SW_BM, mt);
       bool ok = true;
       for (int kb = 0; kb < num_kb && ok; ++kb) {
         const int s = kb % STAGES;
-        ok = mbar_wait(&sm.full[s], (kb / STAGES) & 1, abort_flag, 12, &g_tc_status);
+        ok = __all_sync(0xffffffffu, mbar_wait(&sm.full[s], (kb / STAGES) & 1, abort_flag, 12, &g_tc_status));
         if (!ok) break;
         tc_fence_after();
         const uint64_t da = make_smem_desc(smem_u32(sm.w[s]));
         const uint64_t db = make_smem_desc(smem_u32(sm.x[s]));
 #pragma unroll
-        for (int k = 0; k < SW_BK / 16; ++k) tc_mma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-        tc_commit(&sm.empty[s]);
+        for (int k = 0; k < SW_BK / 16; ++k) tc_mma_bf16_elect(tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+        tc_commit_elect(&sm.empty[s]);
       }
-      if (ok) tc_commit(&sm.acc_full);
+      if (ok) tc_commit_elect(&sm.acc_full);
     }
   } else {
     // ---- epilogue: lane = weight row, columns = tokens ---------------------------------------------
