@@ -180,15 +180,22 @@ extern "C" void qe_gemm_tc_swap_clear_status() {
   cudaMemcpyToSymbol(g_tc_status, &v, sizeof(int));
 }
 
-// 1 <= M <= 256.  Returns 0 when run, 1 when refused (qe_last_error says why), 2 on a launch error.
-extern "C" int qe_linear_tcgen05_swap(const void* x, const void* w, void* out, int M, int N, int K, int out_mode,
+int qe_gemm_tc_stream(const void* x, const void* w, void* out, int M, int N, int K, int out_f32, int act, bool glu, cudaStream_t stream);
+
+// form 0: 128 weight rows a CTA (this file), 1 <= M <= 256.  form 1: 64 weight rows a CTA (gemm_tcgen05_stream.cu), M <= 64.  form
+// 2: the same over stacked weights w [2 N, K], out[M, N] = glu(x · w[:N]^T, x · w[N:]^T) in bfloat16, glu_act as glu_fast takes it.
+// Returns 0 when run, 1 when refused (qe_last_error says why), 2 on a launch error.
+extern "C" int qe_linear_tcgen05_swap(const void* x, const void* w, void* out, int M, int N, int K, int out_mode, int form, int glu_act,
                                       cudaStream_t stream) {
   const int out_f32 = out_mode & 1, act = out_mode >> 1;       // (the activation of the sums: common.cuh)
   if (act < 0 || act > QE_ACT_MAX) QE_REFUSE("linear_tcgen05_swap: unknown activation %d", act);
+  if (form < 0 || form > 2 || (form == 2 && out_mode)) QE_REFUSE("linear_tcgen05_swap: form %d, output mode %d", form, out_mode);
   if (M <= 0 || N <= 0) return 0;
-  if (M > 256) QE_REFUSE("linear_tcgen05_swap: M = %d is above 256", M);
+  if (M > (form ? 64 : 256)) QE_REFUSE("linear_tcgen05_swap: M = %d is above %d", M, form ? 64 : 256);
   if (K <= 0 || K % 8) QE_REFUSE("linear_tcgen05_swap: K = %d is not a positive multiple of 8", K);
-  if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) QE_REFUSE("linear_tcgen05_swap: operands must be 16-byte aligned");
+  // (the forms of 64 rows store element by element)
+  if (((uintptr_t)x | (uintptr_t)w | (form ? 0 : (uintptr_t)out)) & 15) QE_REFUSE("linear_tcgen05_swap: operands must be 16-byte aligned");
+  if (form) return qe_gemm_tc_stream(x, w, out, M, N, K, out_f32, form == 2 ? glu_act : act, form == 2, stream);
   if (M <= 64) return launch_swap<64, 8>(x, w, out, M, N, K, out_f32, stream, act);
   if (M <= 128) return launch_swap<128, 6>(x, w, out, M, N, K, out_f32, stream, act);
   return launch_swap<256, 4>(x, w, out, M, N, K, out_f32, stream, act);

@@ -35,6 +35,13 @@ SPLITK_MAX_CLUSTERS_OF_8 = 8   # clusters of 8 CTAs at most (16 of them, 2 048 w
                                # cluster needs its SMs in one part of the GPU)
 SWAP_MIN_M = 17         # rows from which, up to SMALL_M_MAX, wide products go to the swapped tcgen05 kernel
 SWAP_MIN_N = 3072       # weight rows from which it has enough CTAs (one per 128) to pull the weights fast enough
+STREAM = True              # up to some tens of rows against very many weight rows: 64 of them a CTA, two or three CTAs per SM (gemm_tcgen05_stream.cu)
+STREAM_MAX_M = 32
+STREAM_MIN_N = 16384       # weight rows from which it serves up to 16 rows (fewer CTAs do not fill the SMs' loads) ...
+STREAM_WIDE_MIN_N = 65536  # ... and up to STREAM_MAX_M (several rounds of CTAs)
+STREAM_GLU_MAX_M = 64      # rows up to which the gate/up product with the activation in that kernel's epilogue serves ...
+STREAM_GLU_MIN_N = 6144    # ... from so many stacked weight rows on where the other kernels would need a launch for the activation,
+STREAM_GLU_FEW_MIN_N = 10240   # and from so many on up to SWIGLU_SMALL_MAX_M rows, where the weight-streaming product forms it too
 SWIGLU_FUSED = True     # SiLU-mul in the epilogue of the gate/up product where the CTA-pair kernel serves it
 TCGEN05_PAIRS = True    # CTA pairs for large products
 PAIR_MIN_TILES = 74     # 256 x 256 tiles from which they are used (one per pair of SMs)
@@ -478,6 +485,20 @@ def _hand_over_next_weights() -> None:
         lib().qe_small_m_prefetch_next(_ptr(w), ctypes.c_ulonglong(w.numel() * w.element_size()))
 
 
+def stream_applies(M: int, N: int, K: int, dtype: torch.dtype) -> bool:
+    """Whether the kernel that gives a CTA 64 weight rows serves this product.  Measured on a B200 (a chain of launches): 151 936
+    x 1 024 at 1, 8, 16 and 28 rows 56 -> 51, 65 -> 53, 79 -> 56 and 64 -> 58 us, x 2 560 128 -> 113, 141 -> 117, 167 -> 120
+    and 132 -> 123; 24 576 x 2 048 23.5 -> 16.9 at one row, 29.3 -> 17.6 at 16; 16 384 x 4 096 32.9 -> 24.9.  Up to 8 rows
+    it loses where its CTAs are a little more than a round of three per SM (32 768 x 1 024: 15.0 -> 15.5; at 16 rows, where
+    the other kernels re-read x for two tiles of tokens, 21.2 -> 16.0)."""
+    if not (STREAM and TCGEN05_ENABLED and dtype == torch.bfloat16 and 1 <= M <= STREAM_MAX_M and K % 8 == 0):
+        return False
+    if M > 16:
+        return N >= STREAM_WIDE_MIN_N
+    rounds = -(-N // 64) / (3 * TC_TARGET_CTAS)
+    return N >= STREAM_MIN_N and (M > 8 or not 1 < rounds < 1.5)
+
+
 def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = None) -> None:
     """out[M, N] = x[M, K] · w[N, K]^T, float32 accumulation; out in x's dtype or float32.
     ``x`` may be a NormedInput (see there).  ``activation`` (``ACTIVATIONS``) is applied to the float32 sums in the
@@ -498,6 +519,10 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = No
     _need(out.shape == (M, N) and out.dtype in (x.dtype, torch.float32), "linear: out must be [M, N] in x's dtype or float32")
     _need(x.is_contiguous() and w.is_contiguous() and out.is_contiguous(), "linear: operands must be contiguous")
     out_mode = int(out.dtype == torch.float32) | act << 1
+    if stream_applies(M, N, K, x.dtype):
+        # very many weight rows (a vocabulary): all SMs stream them, 64 a CTA
+        _check(lib().qe_linear_tcgen05_swap(_ptr(x), _ptr(w), _ptr(out), M, N, K, out_mode, 1, 0, _stream()), "linear")
+        return
     splits = splitk_splits(M, N, K, x.dtype)
     if splits:
         linear_splitk(x, w, out, splits, activation=activation)
@@ -505,7 +530,7 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = No
     if (x.dtype == torch.bfloat16 and SWAP_MIN_M <= M <= SMALL_M_MAX and N >= SWAP_MIN_N and K % 8 == 0
             and TCGEN05_ENABLED):
         # some tens of rows and many weight rows: the weights on the 128-row side of tcgen05.mma
-        _check(lib().qe_linear_tcgen05_swap(_ptr(x), _ptr(w), _ptr(out), M, N, K, out_mode, _stream()), "linear")
+        _check(lib().qe_linear_tcgen05_swap(_ptr(x), _ptr(w), _ptr(out), M, N, K, out_mode, 0, 0, _stream()), "linear")
         return
     if x.dtype == torch.bfloat16 and M <= SMALL_M_MAX and K % 8 == 0:
         # a few rows: stream every weight once through the tensor cores
@@ -600,6 +625,36 @@ def linear_swiglu_small(x, w_gate_up: torch.Tensor, out: torch.Tensor, activatio
     _hand_over_next_weights()
     _check(lib().qe_linear_small_m_swiglu(_ptr(x), _ptr(w_gate_up), _ptr(out), M, I, K, gate_code(activation), _stream()),
            "linear_swiglu_small")
+
+
+def swiglu_stream_applies(M: int, I: int, K: int, dtype: torch.dtype) -> bool:
+    """Whether the gate/up product of up to 64 rows forms the activation in the epilogue of the kernel that gives a CTA 64 weight
+    rows (``linear_swiglu_stream``).  Measured on a B200 (a chain of launches, against the weight-streaming product up to 16
+    rows and a tcgen05 product and the activation's launch beyond): 19 456 x 2 560 25.2 -> 17.2 us at 8 rows, 30.0 -> 17.4 at
+    16, 29.7 -> 18.1 at 28; 12 288 x 2 048 11.5 -> 10.6, 13.4 -> 10.7, 13.6 -> 11.2, at 64 rows 15.1 -> 12.5; 6 144 x 1 024
+    3.8 -> 5.5 and 5.0 -> 5.7, but 7.1 -> 6.3 at 28 rows and 8.1 -> 7.2 at 64.  A CTA walks all of K (0.27 us for 128 of it), so
+    it loses where K is long against the rows (6 144 x 4 096 at 28 rows 13.5 -> 15.9), and up to 8 rows where K is short
+    (16 384 x 1 024 7.1 -> 8.2)."""
+    if not (STREAM and TCGEN05_ENABLED and dtype == torch.bfloat16 and 1 <= M <= STREAM_GLU_MAX_M and K % 8 == 0):
+        return False
+    few = M <= SWIGLU_SMALL_MAX_M
+    return 2 * I >= (STREAM_GLU_FEW_MIN_N if few else STREAM_GLU_MIN_N) and 2 * I >= 3 * K and (M > 8 or K >= 2048)
+
+
+def linear_swiglu_stream(x, w_gate_up: torch.Tensor, out: torch.Tensor, activation: str = "silu") -> None:
+    """out[M, I] = act(x · w_gate^T) * (x · w_up^T) over the stacked weights, up to 64 rows: the activation is formed on the
+    float32 sums in the product's epilogue."""
+    if isinstance(x, NormedInput):
+        x = x.materialize()
+    M, K = x.shape
+    I = w_gate_up.shape[0] // 2
+    _need(x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and w_gate_up.shape == (2 * I, K) and K % 8 == 0,
+          "linear_swiglu_stream: bfloat16 operands, w [2 I, K] with K a multiple of 8")
+    _need(out.shape == (M, I) and out.dtype == torch.bfloat16 and M <= STREAM_GLU_MAX_M,
+          f"linear_swiglu_stream: out must be bfloat16 [M, I] with M <= {STREAM_GLU_MAX_M}")
+    _need(x.is_contiguous() and w_gate_up.is_contiguous() and out.is_contiguous(), "linear_swiglu_stream: operands must be contiguous")
+    _check(lib().qe_linear_tcgen05_swap(_ptr(x), _ptr(w_gate_up), _ptr(out), M, I, K, 0, 2, gate_code(activation), _stream()),
+           "linear_swiglu_stream")
 
 
 QKV_ROPE_FUSED = True       # many rows: per-head norm, rotation and cache write in the epilogue of the QKV product
@@ -781,9 +836,9 @@ def tcgen05_status() -> int:
     """0 if no bounded wait of the tcgen05 product kernels ever ran out; else the code of the first
     that did (1: a shared-memory slot never came free, 2: TMA bytes never landed, 3: the
     accumulator never completed, 4: an accumulator was never read out; 11-13: the same as 1-3 in the
-    kernel for some tens of rows, 21-23 in its form that shares K within a cluster).  Synchronises the device."""
+    kernel for some tens of rows, 21-23 in its form that shares K within a cluster, 31-33 in its form of 64 weight rows a CTA).  Synchronises the device."""
     return (int(lib().qe_gemm_tc_status()) or int(lib().qe_gemm_tc_swap_status()) or int(lib().qe_gemm_tc_pair_status())
-            or int(lib().qe_gemm_tc_splitk_status()))
+            or int(lib().qe_gemm_tc_splitk_status()) or int(lib().qe_gemm_tc_stream_status()))
 
 
 class DeviceWaitTimeout(RuntimeError):
@@ -791,7 +846,7 @@ class DeviceWaitTimeout(RuntimeError):
     the step produced is not to be trusted."""
 
 
-_STATUS_WORDS = ("qe_gemm_tc", "qe_gemm_tc_swap", "qe_gemm_tc_pair", "qe_gemm_tc_splitk", "qe_flash_attention_tc",
+_STATUS_WORDS = ("qe_gemm_tc", "qe_gemm_tc_swap", "qe_gemm_tc_pair", "qe_gemm_tc_splitk", "qe_gemm_tc_stream", "qe_flash_attention_tc",
                  "qe_flash_attention", "qe_decode_attention_mma", "qe_small_m", "qe_latent_decode", "qe_moe_tc", "qe_latent_attention_tc",
                  "qe_head_linear_tc")
 

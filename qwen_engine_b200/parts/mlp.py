@@ -59,6 +59,14 @@ class SwiGLU(FeedForward):
             ops.linear_swiglu(x, self.w_gate_up, act, self.activation)
             ops.linear(act, self.w_down, out)
             return
+        if ops.swiglu_stream_applies(T, I, self.hidden_size, ctx.dtype):
+            # up to some tens of rows and many weight rows: the activation comes out of the product's epilogue too
+            act = ctx.arena.alloc((T, I), ctx.dtype)
+            ops.linear_swiglu_stream(x, self.w_gate_up, act, self.activation)
+            ops.prefetch_next(step_hint(ctx, "weights_after_ffn"))
+            ops.linear(act, self.w_down, out)
+            ops.prefetch_next(None)
+            return
         if ops.swiglu_small_applies(T, I, self.hidden_size, ctx.dtype):
             # a few rows: the product that streams the gate and up weights forms the activation itself
             act = ctx.arena.alloc((T, I), ctx.dtype)

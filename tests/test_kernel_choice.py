@@ -53,3 +53,15 @@ def test_other_types_and_many_rows_are_not_for_that_kernel():
     assert ops.splitk_splits(32, 1024, 2048, torch.float32) == 0
     assert ops.splitk_splits(65, 1024, 2048, BF) == 0
     assert ops.splitk_splits(32, 1024, 2052, BF) == 0          # K must be a multiple of 8
+
+
+def test_very_many_weight_rows_go_64_to_a_cta():
+    for K in (1024, 2048, 2560):
+        assert all(ops.stream_applies(M, 151936, K, BF) for M in (1, 8, 16, 32)) and not ops.stream_applies(33, 151936, K, BF)
+    assert not ops.stream_applies(8, 32768, 1024, BF) and ops.stream_applies(9, 32768, 1024, BF) and not ops.stream_applies(17, 32768, 1024, BF)
+    assert not ops.stream_applies(8, 151936, 1024, torch.float32) and not ops.stream_applies(8, 151936, 1020, BF)
+    assert not any(ops.stream_applies(M, N, K, BF) for M in (1, 16, 32) for name in ("0.6b", "1.7b") for N, K in _products(name).values())
+    glu = lambda M, name: ops.swiglu_stream_applies(M, SIZES[name][1], SIZES[name][0], BF)
+    assert all(glu(M, "4b") and glu(M, "1.7b") for M in (1, 8, 16, 17, 64)) and not glu(65, "4b")
+    assert not glu(8, "0.6b") and not glu(16, "0.6b") and glu(17, "0.6b") and glu(64, "0.6b")
+    assert not ops.swiglu_stream_applies(28, 3072, 4096, BF), "K too long for a CTA alone"

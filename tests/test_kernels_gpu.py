@@ -186,6 +186,50 @@ def test_linear_tcgen05_swapped(M, N, K, out_f32, monkeypatch):
     _close(got, want, torch.bfloat16, scale=float(want.float().abs().max()))
 
 
+@pytest.mark.parametrize("M", [1, 8, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(64, 64), (63, 8), (130, 200), (16391, 136), (28480, 1032)])
+@pytest.mark.parametrize("out_f32", [False, True])
+def test_linear_tcgen05_stream(M, N, K, out_f32, monkeypatch):
+    """64 weight rows a CTA, up to 32 rows: edges in M, N (an odd number of rows, one CTA more than three per SM) and K (less
+    than half a stage, one half of the last one missing)."""
+    monkeypatch.setattr(ops, "STREAM_MIN_N", 1)
+    monkeypatch.setattr(ops, "STREAM_WIDE_MIN_N", 1)
+    assert ops.stream_applies(M, N, K, torch.bfloat16) or (N == 28480 and M <= 8)
+    x = _randn((M, K), torch.bfloat16, 18)
+    w = _randn((N, K), torch.bfloat16, 19, 0.1)
+    odt = torch.float32 if out_f32 else torch.bfloat16
+    want = torch.empty(M, N, dtype=odt)
+    ref_ops.linear(x, w, want)
+    got = torch.full((M + 1, N), float("nan"), dtype=odt, device=DEV)
+    ops.linear(x.to(DEV), w.to(DEV), got[:M])
+    torch.cuda.synchronize()
+    assert ops.tcgen05_status() == 0 and got[M].isnan().all()
+    _close(got[:M], want, torch.bfloat16, scale=float(want.float().abs().max()))
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 31, 33, 64])
+@pytest.mark.parametrize("I,K", [(32, 64), (45, 136), (3072, 1024), (7168, 72)])
+@pytest.mark.parametrize("activation", ["silu", "gelu_tanh", (ops.LIMITED_GLU, 1.5)])
+def test_linear_swiglu_stream(M, I, K, activation):
+    """The gate/up product whose CTAs hold 32 rows of each, with the activation on the float32 sums; edges in M, I and K."""
+    x = _randn((M, K), torch.bfloat16, 36)
+    w = _randn((2 * I, K), torch.bfloat16, 37, 0.1)
+    g = x.float() @ w[:I].float().t()
+    u = x.float() @ w[I:].float().t()
+    if activation == "silu":
+        want = g / (1 + torch.exp(-g)) * u
+    elif activation == "gelu_tanh":
+        want = torch.nn.functional.gelu(g, approximate="tanh") * u
+    else:
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        want = g * torch.sigmoid(1.702 * g) * (u + 1)
+    got = torch.full((M + 1, I), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.linear_swiglu_stream(x.to(DEV), w.to(DEV), got[:M], activation)
+    torch.cuda.synchronize()
+    assert ops.tcgen05_status() == 0 and got[M].isnan().all()
+    _close(got[:M], want, torch.bfloat16, scale=float(want.abs().max()), tol16=1e-2)
+
+
 @pytest.mark.parametrize("M", [1, 9, 17, 33, 64])
 @pytest.mark.parametrize("N,K,splits", [(1024, 2048, 8), (1024, 3072, 8), (1000, 1032, 4), (132, 200, 2), (4096, 1024, 4),
                                         (256, 192, 8), (6144, 1024, 2), (2560, 4096, 4)])
