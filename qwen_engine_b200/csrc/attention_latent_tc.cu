@@ -283,6 +283,9 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   }
 }
 
+// Shared memory of a CTA: it takes all of an SM's tensor memory, so it leaves no other CTA that wants some room beside it, however
+// small D is (tcgen05.cuh: a CTA of 81 KB, D up to 64, could wait for columns that a product behind it held, which waited
+// for it).
 static int lt_smem_of(int D, int* col_blocks, int* slots) {
   const int cb = (D + 63) / 64;
   const int q = cb * LT_ROWS * 128, slot = cb * LT_BN * 128, limit = 224 * 1024;
@@ -290,7 +293,16 @@ static int lt_smem_of(int D, int* col_blocks, int* slots) {
   n = n > LT_MAX_SLOTS ? LT_MAX_SLOTS : n;
   *col_blocks = cb;
   *slots = n;
-  return q + n * slot + 1024;
+  const int smem = q + n * slot + 1024;
+  return smem > TC_SMEM_ALONE ? smem : TC_SMEM_ALONE;
+}
+static_assert(tc_room_for_all(TC_SMEM_ALONE, 512), "alone among the kernels with tensor memory");
+
+// What a launch over cache rows of D channels asks for, and the least that leaves no other CTA with tensor memory room on the SM.
+extern "C" int qe_latent_attention_tc_smem(int D, int* alone) {
+  int cb, n;
+  *alone = TC_SMEM_ALONE;
+  return lt_smem_of(D, &cb, &n);
 }
 
 extern "C" int qe_latent_attention_tc_status() {

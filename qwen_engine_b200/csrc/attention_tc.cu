@@ -970,6 +970,7 @@ extern "C" int qe_flash_attention_tc(const void* q, long q_stride, int T, const 
               scale * 1.4426950408889634f, window, Hq, Hkv, page_shift, slopes, 1.f / scale,
               softcap > 0.f ? scale / softcap : 0.f, softcap > 0.f ? softcap / scale : 0.f, sinks, v_shift, value_blocks};
   const size_t smem = sizeof(AtSmem) + 1024;
+  static_assert(tc_room_for_all(sizeof(AtSmem) + 1024, AT_TMEM_COLS), "tensor memory for every CTA that finds room on an SM");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(flash_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -237,6 +237,7 @@ static int launch_tc(const void* x, const void* w, void* out, int M, int N, int 
   CUtensorMap map_x, map_w;
   if (!get_map(x, M, K, TC_BM, &map_x) || !get_map(w, N, K, BN, &map_w)) return 1;
   const size_t smem = sizeof(TcSmem<BN, STAGES>) + 1024;
+  static_assert(tc_room_for_all(sizeof(TcSmem<BN, STAGES>) + 1024, 2 * BN), "tensor memory for every CTA that finds room on an SM");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<__nv_bfloat16, BN, STAGES, false, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -578,6 +578,7 @@ static int launch_pair(const void* x, const void* w, void* out, int M, int N, in
   const size_t smem = sizeof(PrSmem<BN, STAGES, ROPE>) + 1024 - 256;
 #else
   const size_t smem = sizeof(PrSmem<BN, STAGES, ROPE>) + 1024;
+  static_assert(tc_room_for_all(sizeof(PrSmem<BN, STAGES, ROPE>) + 1024, 2 * BN), "tensor memory for every CTA that finds room on an SM");
 #endif
   static bool configured = false;
   if (!configured) {

@@ -188,6 +188,7 @@ static int launch_stream(const void* x, const void* w, void* out, int M, int N, 
     if (!qe_tensor_map_bf16(x, 2, dims, strides, box, &map_x)) return 1;
   }
   const size_t smem = sizeof(SrSmem<BT, STAGES>) + 1024;
+  static_assert(tc_room_for_all(sizeof(SrSmem<BT, STAGES>) + 1024, BT < 32 ? 32 : BT), "tensor memory for every CTA that finds room on an SM");
   static const cudaError_t configured =
       cudaFuncSetAttribute(gemm_tcgen05_stream_kernel<TOut, BT, STAGES, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (configured != cudaSuccess) QE_REFUSE("linear_tcgen05_stream: shared memory %zu: %s", smem, cudaGetErrorString(configured));

@@ -154,6 +154,7 @@ static int launch_swap(const void* x, const void* w, void* out, int M, int N, in
     if (!qe_tensor_map_bf16(x, 2, dims, strides, box, &map_x)) return 1;
   }
   const size_t smem = sizeof(SwSmem<BT, STAGES>) + 1024;
+  static_assert(tc_room_for_all(sizeof(SwSmem<BT, STAGES>) + 1024, BT < 32 ? 32 : BT), "tensor memory for every CTA that finds room on an SM");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_swap_kernel<__nv_bfloat16, BT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

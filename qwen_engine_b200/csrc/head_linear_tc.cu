@@ -173,6 +173,7 @@ static int launch_head_linear_tc(const void* x, long ldx, long ldx_h, const void
     if (!qe_tensor_map_bf16(w, 3, dims, strides, box, &map_w)) return 1;
   }
   const size_t smem = sizeof(HtSmem<BN>) + 1024;
+  static_assert(tc_room_for_all(sizeof(HtSmem<BN>) + 1024, BN <= 64 ? 128 : BN <= 128 ? 256 : 512), "tensor memory for every CTA that finds room on an SM");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(head_linear_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

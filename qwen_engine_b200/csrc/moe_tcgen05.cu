@@ -262,6 +262,7 @@ extern "C" int qe_moe_tc(const void* rows, const void* w, const int* offsets, vo
     if (!qe_tensor_map_bf16(w, 2, dims, strides, box, &map_w)) return 1;
   }
   const size_t smem = sizeof(MtSmem) + 1024;
+  static_assert(tc_room_for_all(sizeof(MtSmem) + 1024, 2 * MT_BN), "tensor memory for every CTA that finds room on an SM");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(moe_tcgen05_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -124,6 +124,15 @@ __device__ __forceinline__ void tc_st_32x32b_x32(uint32_t taddr, const uint32_t 
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
+// tcgen05.alloc waits, without a limit, until the columns are free, and the kernels of a stream overlap both ways: a CTA may
+// meet on its SM one of a later kernel that already holds columns and waits for this kernel's end.  So the columns of all
+// CTAs that find room on an SM together must fit its 512.  Every kernel that allocates takes at least TC_SMEM_LEAST of
+// shared memory (three such CTAs per SM at most) and at most 128 columns, or so much shared memory that none of the others
+// finds room beside it (1 KB of an SM's shared memory is the system's for each CTA).
+#define TC_SMEM_SM (228 * 1024)
+#define TC_SMEM_LEAST (60 * 1024)
+#define TC_SMEM_ALONE (TC_SMEM_SM - 2 * 1024 - TC_SMEM_LEAST + 16)
+constexpr bool tc_room_for_all(size_t smem, uint32_t cols) { return smem >= TC_SMEM_LEAST && (cols <= 128 || smem >= TC_SMEM_ALONE); }
 // One warp allocates `cols` columns (a power of two, 32..512) of tensor memory and writes their base
 // address to shared memory; the same warp frees them.
 __device__ __forceinline__ void tc_alloc(uint32_t* result_in_smem, uint32_t cols) {

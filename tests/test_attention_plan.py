@@ -134,3 +134,15 @@ def test_contexts_are_cut_by_length_only_where_they_are_unequal():
     assert splits(ragged * 2 + ragged[:8]) == 74 and type(splits(ragged * 3)) is int
     beside = ops.plan_attention([512] + [1] * 15, [0] + [150 + 130 * i for i in range(15)], 16, (geo,), bf)
     assert len(_items(beside, "fa0_items")) == beside["fa0_info"][0] == 37
+
+
+def test_latent_attention_shares_an_sm_with_no_other_tensor_memory():
+    """Its CTAs take all 512 columns of tensor memory, for which a CTA waits without a limit; a product behind it that held some on
+    the same SM would itself wait for this kernel's end.  Whatever the cache row's size, a launch asks for so much shared memory
+    that the smallest of those kernels (60 KB) does not fit beside it in an SM's 228 KB, 1 KB of which goes with each CTA."""
+    import ctypes
+    for D in range(16, 257, 16):
+        alone = ctypes.c_int()
+        smem = int(ops.lib().qe_latent_attention_tc_smem(D, ctypes.byref(alone)))
+        assert alone.value <= smem <= 225 * 1024
+        assert smem + 1024 + 60 * 1024 + 1024 > 228 * 1024, D
