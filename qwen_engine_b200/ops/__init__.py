@@ -12,6 +12,7 @@ import ctypes
 import heapq
 import os
 import struct
+import weakref
 from typing import Optional
 
 import torch
@@ -871,8 +872,9 @@ def clear_device_status() -> None:
         return
     for name in _STATUS_WORDS:
         getattr(lib(), name + "_clear_status")()
-    for t in _merge_counter_tensors.values():
-        t.zero_()
+    for arena in list(_arenas_with_counters):
+        for t in arena.counters.values():
+            t.zero_()
 
 
 def check_device_status() -> None:
@@ -1276,18 +1278,18 @@ def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype
 
 
 _MERGE_COUNTERS = 1 << 16
-_merge_counter_tensors: dict = {}
+_arenas_with_counters: "weakref.WeakSet" = weakref.WeakSet()
 
 
-def _merge_counters(device, kernel: str = "fa") -> torch.Tensor:
+def _merge_counters(arena, kernel: str = "fa") -> torch.Tensor:
     """Zeroed ints, one per (part, kv head), that an attention kernel uses to find the CTA that finishes a
-    split context last (it merges the parts and sets its counter back to zero).  One tensor per device
-    and kernel for the life of the process, so that its address is the same in every captured step."""
-    key = (torch.device(device).index, kernel)
-    t = _merge_counter_tensors.get(key)
+    split context last (it merges the parts and sets its counter back to zero).  They belong to the arena that
+    holds the parts and live as long as it, one tensor per kernel: the address is the same in every captured step, and
+    two step functions whose launches overlap (two engines on two streams) never count into the same words."""
+    t = arena.counters.get(kernel)
     if t is None:
-        t = torch.zeros(_MERGE_COUNTERS, dtype=torch.int32, device=device)
-        _merge_counter_tensors[key] = t
+        t = arena.counters[kernel] = torch.zeros(_MERGE_COUNTERS, dtype=torch.int32, device=arena.device)
+        _arenas_with_counters.add(arena)
     return t
 
 
@@ -1404,7 +1406,7 @@ def paged_attention(qkv: torch.Tensor, kv_pages: torch.Tensor, block_tables: tor
             _need(2 * tc_parts * Hkv * VB <= _MERGE_COUNTERS, "paged_attention: too many parts")   # (two counters a tile and kv head)
             part_acc = ctx.arena.alloc((tc_parts * Hkv * VB * tc_rows, D), torch.float32)
             part_ml = ctx.arena.alloc((tc_parts * Hkv * VB * tc_rows, 2), torch.float32)
-            counters = _merge_counters(qkv.device, "tc")
+            counters = _merge_counters(ctx.arena, "tc")
         _check(lib().qe_flash_attention_tc(
             _ptr(qkv), ctypes.c_long(qkv.stride(0)), T, _ptr(kv_pages), int(kv_pages.shape[0]), _ptr(block_tables),
             int(block_tables.shape[1]), _ptr(tc_items), tc_items.numel() // FLASH_ITEM_INTS,
@@ -1426,7 +1428,7 @@ def paged_attention(qkv: torch.Tensor, kv_pages: torch.Tensor, block_tables: tor
         if n_parts:
             part_acc = ctx.arena.alloc((S * n_parts * Hkv * part_rows, D), torch.float32)
             part_ml = ctx.arena.alloc((S * n_parts * Hkv * part_rows, 2), torch.float32)
-        counters = _merge_counters(qkv.device) if 0 < S * n_parts * Hkv <= _MERGE_COUNTERS else None
+        counters = _merge_counters(ctx.arena) if 0 < S * n_parts * Hkv <= _MERGE_COUNTERS else None
         if (planes == 1 and softcap <= 0.0 and latent_decode_supported((Hq, Hkv, D, window, False, 1), qkv.dtype)
                 and (max_rows <= 16 or ctx.max_q_len == 1) and qkv.stride(0) % 8 == 0
                 and n_parts * -(-max_rows // 16) <= _MERGE_COUNTERS):
@@ -1437,7 +1439,7 @@ def paged_attention(qkv: torch.Tensor, kv_pages: torch.Tensor, block_tables: tor
                 cluster = 0
             _check(lib().qe_latent_decode(
                 _ptr(qkv), ctypes.c_long(qkv.stride(0)), _ptr(kv_pages), _ptr(block_tables), int(block_tables.shape[1]), _ptr(items), n_items,
-                _ptr(out), _ptr(part_acc), _ptr(part_ml), int(part_rows), _ptr(_merge_counters(qkv.device)), int(max_rows), cluster,
+                _ptr(out), _ptr(part_acc), _ptr(part_ml), int(part_rows), _ptr(_merge_counters(ctx.arena) if n_parts else None), int(max_rows), cluster,
                 ctypes.c_float(scale), int(window), Hq, D, int(value_dim or D), int(kv_pages.shape[3]), _ptr(sinks), _stream()), "latent_decode")
             return
         # every request in the same few parts: the parts of a request form a cluster and meet on chip

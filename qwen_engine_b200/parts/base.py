@@ -44,6 +44,9 @@ class Arena:
     buffer grows at the next ``reset()``.  Steps repeat the same allocations, so
     the views into the buffer are kept by (offset, shape, dtype) and handed out
     again: making a view costs more host time than a launch.
+
+    ``counters``: what the attention kernels count a split context's finished parts by (``ops._merge_counters``); a launch
+    leaves them at zero, and they outlive ``reset()``.
     """
 
     ALIGN = 256
@@ -59,6 +62,7 @@ class Arena:
         self._overflow: list[torch.Tensor] = []
         self._overflow_bytes = 0
         self._views: dict = {}
+        self.counters: dict[str, torch.Tensor] = {}
 
     def reset(self) -> None:
         if self._overflow:

@@ -64,3 +64,46 @@ def test_a_remembered_view_is_not_handed_out_over_step_memory():
     s = ar.alloc_step((512,), torch.float32)                   # 2 KB at the far end
     again = ar.alloc((768,), torch.float32)                    # the remembered view would run into it
     assert not _overlap(again, s)
+
+
+def test_finished_parts_are_counted_where_the_parts_lie(monkeypatch):
+    """Two step functions (two engines on two streams) never count into the same words, and one step function's counters stay
+    where they are (captured steps hold their address); those that a kernel gave up over are set back to zero.  The counters
+    that a decode step's launch is given are looked at; nothing is launched."""
+    import ctypes
+    from types import SimpleNamespace
+
+    from qwen_engine_b200 import ops
+    from qwen_engine_b200.engine.runner import ModelRunner
+    R, Hq, Hkv, D, P = 12, 16, 8, 128, 16
+    ctx_lens, geo, bf = [100 + 150 * i for i in range(R)], (Hq, Hkv, D, 0), torch.bfloat16
+    plan = ops.plan_attention([1] * R, ctx_lens, P, (geo,), bf, uniform_splits={geo: ops.TotalParts(37)})
+    seen = []
+
+    class Library:
+        def __getattr__(self, name):
+            def call(*args):
+                if name == "qe_decode_attention_mma":
+                    seen.append(args[12].value)
+                return 0
+            return call
+    monkeypatch.setattr(ops, "lib", Library)
+    monkeypatch.setattr(ops, "_lib", object())
+    monkeypatch.setattr(ops, "_ptr", lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr()))
+    monkeypatch.setattr(ops, "_stream", lambda: ctypes.c_void_p(0))
+    arenas = [Arena("cpu", 1 << 16), Arena("cpu", 1 << 16)]
+    for _ in range(2):
+        for arena in arenas:
+            arena.reset()
+            dev = {"plan_" + k: torch.tensor(v, dtype=torch.int32) for k, v in plan.items()}
+            ctx = SimpleNamespace(cu_q=torch.arange(R + 1, dtype=torch.int32), ctx_lens=torch.tensor(ctx_lens, dtype=torch.int32),
+                                  q_lens_host=[1] * R, ctx_lens_host=ctx_lens, max_q_len=1, arena=arena,
+                                  attn_plan=ModelRunner._device_plan(plan, dev, (geo,)))
+            ops.paged_attention(torch.zeros(R, (Hq + 2 * Hkv) * D, dtype=bf), torch.zeros(2, 2, Hkv, P, D, dtype=bf),
+                                torch.zeros(R, 2, dtype=torch.int32), ctx, torch.zeros(R, Hq * D, dtype=bf), 0.1, 0, Hq, Hkv, D)
+    assert len(seen) == 4 and all(seen)
+    assert seen[:2] == seen[2:] and seen[0] != seen[1]
+    assert all((a.counters["fa"] == 0).all() for a in arenas)
+    arenas[1].counters["fa"][5] = 2
+    ops.clear_device_status()
+    assert (arenas[1].counters["fa"] == 0).all()

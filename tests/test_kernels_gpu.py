@@ -10,6 +10,7 @@ import torch
 
 import ref_ops
 from qwen_engine_b200 import ops
+from qwen_engine_b200.parts.base import Arena
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -552,12 +553,14 @@ def _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed, spike=
                 ctx=torch.tensor(ctx_lens, dtype=torch.int32), T=T)
 
 
-def _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, fn, dev, flash=True, uniform=None):
-    """Run one implementation.  On the GPU ``flash`` lets the step's plan carry the tensor-core
+def _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, fn, dev, flash=True, uniform=None, arena=None):
+    """Run one implementation (``arena``: with that scratch memory, and the counters that belong to it).  On the GPU ``flash`` lets the step's plan carry the tensor-core
     kernel's work items (used when the kernel takes the geometry); without it the generic kernel runs.
     ``uniform``: every request's context in that many parts, as in a decode step replayed from a graph."""
     from qwen_engine_b200.engine.runner import ModelRunner
-    from qwen_engine_b200.parts.base import Arena
+    if arena is None:
+        arena = Arena(dev)
+    arena.reset()
     scale = 1.0 / math.sqrt(D)
     geos = ((Hq, Hkv, D, window),) if (flash and dev != "cpu") else ()
     plan = ops.plan_attention(list(q_lens), list(ctx_lens), P, geos, dtype,
@@ -565,7 +568,7 @@ def _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, fn, dev
     devplan = ModelRunner._device_plan(
         plan, {"plan_" + k: torch.tensor(v, dtype=torch.int32, device=dev) for k, v in plan.items()}, geos)
     ctx = SimpleNamespace(cu_q=case["cu_q"].to(dev), ctx_lens=case["ctx"].to(dev), attn_plan=devplan,
-                          q_lens_host=list(q_lens), ctx_lens_host=list(ctx_lens), arena=Arena(dev))
+                          q_lens_host=list(q_lens), ctx_lens_host=list(ctx_lens), arena=arena)
     out = torch.zeros(case["T"], Hq * D, dtype=dtype, device=dev)
     fn(case["qkv"].to(dev), case["cache"].to(dev), case["table"].to(dev), ctx, out, scale, window, Hq, Hkv, D)
     if dev != "cpu":
@@ -713,11 +716,13 @@ def test_decode_attention_parts_by_length(Hq, Hkv, P, window, ctx_lens, total, d
     q_lens = [1] * len(ctx_lens)
     case = _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed=61)
     want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ref_ops.paged_attention, "cpu")
+    arena = Arena(DEV)
     for _ in range(2):                                  # (the second launch finds the counters as the first left them)
-        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, uniform=ops.TotalParts(total))
+        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, uniform=ops.TotalParts(total),
+                             arena=arena)
         assert ops.last_attention_kernel == "decode_attention_mma"
         _close(got, want, dtype)
-    assert int(ops._merge_counters(torch.device(DEV)).abs().max()) == 0
+    assert int(arena.counters["fa"].abs().max()) == 0
 
 
 def test_decode_attention_mma_asks_for_the_next_layers_cache(monkeypatch):
@@ -806,8 +811,9 @@ def test_tc_attention_parts(q_lens, ctx_lens):
     assert plan["tc0_info"][0] > 1, "the case must cut tiles into parts"
     case = _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, seed=32)
     want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ref_ops.paged_attention, "cpu")
+    arena = Arena(DEV)
     for _ in range(2):                     # twice: the counters are back at zero after a launch
-        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ops.paged_attention, DEV)
+        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ops.paged_attention, DEV, arena=arena)
         assert ops.tc_attention_status() == 0
         _close(got, want, dtype)
 
@@ -842,8 +848,9 @@ def test_tc_attention_units_one_after_the_other(ctas, Hq, Hkv, P, q_lens, ctx_le
     sched, n = plan["tc0_sched"], plan["tc0_info"][2]
     assert n == min(ctas, units) and sched[0] == n + 1 and sched[n] == len(sched)
     assert sorted(sched[n + 1:]) == list(range(units)), "every unit is run once"
+    arena = Arena(DEV)
     for _ in range(2):                     # twice: the merge counters are back at zero after a launch
-        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV)
+        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, arena=arena)
         assert ops.tc_attention_status() == 0
         assert torch.equal(got, each)
 
