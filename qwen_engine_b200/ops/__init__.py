@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import heapq
+import math
 import os
 import struct
 import weakref
@@ -1076,12 +1077,17 @@ def value_block_size(key_dim: int, value_dim: int) -> tuple[int, int]:
 
 
 class TotalParts(int):
-    """In ``uniform_splits``, in the place of a number of parts per request: the work items of all requests together."""
+    """In ``uniform_splits``, in the place of a number of parts per request: the work items of all requests together.
+    ``shares``: how many of them each request has, where they have been dealt out already (``parts_by_length``)."""
+
+    shares: Optional[list] = None
 
 
-def attended_keys(q_len: int, ctx_len: int, window: int) -> int:
-    """The keys that a request's parts are cut from (from the window's first key tile on)."""
-    return ctx_len + q_len - (max(0, ctx_len - window + 1) // FLASH_BN * FLASH_BN if window else 0)
+def attended_keys(q_lens: list[int], ctx_lens: list[int], window: int) -> list[int]:
+    """The keys that each request's parts are cut from (from the window's first key tile on)."""
+    if not window:
+        return [c + n for n, c in zip(q_lens, ctx_lens)]
+    return [c + n - max(0, c - window + 1) // FLASH_BN * FLASH_BN for n, c in zip(q_lens, ctx_lens)]
 
 
 def parts_by_length(keys: list[int], total: int) -> list[int]:
@@ -1112,8 +1118,51 @@ def parts_for_lengths(geo, keys: list[int], one_each: int) -> Optional[TotalPart
     if not DECODE_PARTS_BY_LENGTH or slots < 1 or len(keys) >= total or total * geo[1] * value_blocks(geo) > _MERGE_COUNTERS:
         return None
     even = sum(keys) / slots
-    longest = max(-(-n // p) for n, p in zip(keys, parts_by_length(keys, total)))
-    return TotalParts(total) if max(longest, even) + DECODE_PART_COST_KEYS < max(one_each, even) else None
+    # below this many keys the longest part has to stay; sums and counts tell most batches apart before anything is dealt out
+    limit = max(one_each, even) - DECODE_PART_COST_KEYS
+    most = math.ceil(limit) - 1
+    if even >= limit or most < 1 or sum([-(-n // most) for n in keys]) > total:
+        return None
+    shares = parts_by_length(keys, total)
+    if max([-(-n // p) for n, p in zip(keys, shares)]) > most:
+        return None
+    parts = TotalParts(total)
+    parts.shares = shares
+    return parts
+
+
+_NO_ROWS = [0, 0, 0, 0, -1] + [0] * (FLASH_ITEM_INTS - 5)        # a work item that holds nothing
+
+
+def _decoded_items(ctx_lens: list[int], parts) -> tuple[list[int], list[int], int]:
+    """The work items, merge items and number of parts of a step of decoded tokens alone, as ``plan_attention`` lays them out:
+    ``parts`` of every request (a number) or of each (a list)."""
+    items: list[int] = []
+    merge: list[int] = []
+    n_parts = 0
+    if parts == 1:
+        for r in sorted(range(len(ctx_lens)), key=ctx_lens.__getitem__, reverse=True):
+            c = ctx_lens[r]
+            items += (r, 0, 0, c + 1, -1, 0, 0, r, 1, c, 0, 0)
+    elif isinstance(parts, int):
+        for r, c in enumerate(ctx_lens):
+            for sp in range(parts):
+                items += (r, 0, 0, 0, n_parts + sp, parts, sp, r, 1, c, 0, 0)
+            merge += (r, 0, n_parts, parts)
+            n_parts += parts
+    else:
+        by_keys: list[tuple[int, tuple]] = []           # (keys of the item, the item)
+        for r, (c, p) in enumerate(zip(ctx_lens, parts)):
+            if p == 1:
+                by_keys.append((c + 1, (r, 0, 0, c + 1, -1, 0, 0, r, 1, c, 0, 0)))
+            else:
+                keys = -(-(c + 1) // p)
+                by_keys += [(keys, (r, 0, 0, 0, n_parts + sp, p, sp, r, 1, c, 0, 0)) for sp in range(p)]
+                n_parts += p
+        by_keys.sort(key=lambda e: e[0], reverse=True)
+        for _, item in by_keys:
+            items += item
+    return items, merge, n_parts
 
 
 def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
@@ -1132,16 +1181,30 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
     ``uniform_splits`` (geometry -> number of parts) fixes the number of parts of every request, or (``TotalParts``) the
     number of work items of all of them, which are then dealt out by length, so that the lists' lengths depend on the
     batch's shape only (for steps replayed from a CUDA graph)."""
-    tiles: list[int] = []
-    for r, n in enumerate(q_lens):
-        for q0 in range(0, n, ATTN_TILE_Q):
-            tiles += [r, q0]
+    decoded = uniform_splits is not None and max(q_lens, default=0) == 1 == min(q_lens, default=0)     # a step of decoded tokens alone
+    if decoded:
+        tiles = [x for r in range(len(q_lens)) for x in (r, 0)]
+    else:
+        tiles = [x for r, n in enumerate(q_lens) for q0 in range(0, n, ATTN_TILE_Q) for x in (r, q0)]
     plan = {"tiles": tiles}
     for gi, geo in enumerate(geometries):
         Hq, Hkv, D, window, biased = split_geometry(geo)
         if not flash_supported(dtype, Hq, Hkv, D):
             continue
         G = Hq // Hkv
+        if decoded:
+            parts = uniform_splits[geo]
+            total = int(parts) if isinstance(parts, TotalParts) else 0
+            if total:
+                parts = parts.shares or parts_by_length(attended_keys(q_lens, ctx_lens, window), total)
+            items, merge, n_parts = _decoded_items(ctx_lens, parts)
+            if total:
+                items += _NO_ROWS * (total - len(items) // FLASH_ITEM_INTS)
+                n_parts = total
+            plan[f"fa{gi}_items"] = items
+            plan[f"fa{gi}_merge"] = merge
+            plan[f"fa{gi}_info"] = [n_parts, G if n_parts else 1, int(G <= 16), G, parts if not total and parts in (2, 4, 8) else 0]
+            continue
         tpt = FLASH_ROWS // G
         latent_tc = latent_tc_supported(geo, dtype, page_size)
         vb = value_blocks(geo)
@@ -1161,10 +1224,13 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
         elif (rest and len(rest) < len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_BESIDE_TC and D == 128
               and geometry_planes(geo) >= 2 and max(q_lens[r] for r in rest) * G <= 16):
             at_most = max(1, FLASH_TARGET_CTAS // base)
-            keys = [attended_keys(q_lens[r], ctx_lens[r], window) for r in rest]
+            keys = attended_keys([q_lens[r] for r in rest], [ctx_lens[r] for r in rest], window)
             items_in_all = parts_for_lengths(geo, keys, max(-(-k // min(-(-k // FLASH_SPLIT), at_most)) for k in keys))
         if items_in_all is not None:
-            shares = dict(zip(rest, parts_by_length([attended_keys(q_lens[r], ctx_lens[r], window) for r in rest], items_in_all)))
+            dealt = items_in_all.shares
+            if dealt is None:
+                dealt = parts_by_length(attended_keys([q_lens[r] for r in rest], [ctx_lens[r] for r in rest], window), items_in_all)
+            shares = dict(zip(rest, dealt))
         for r, (n, c) in enumerate(zip(q_lens, ctx_lens)):
             total = c + n
             if on_tc[r]:
@@ -1205,7 +1271,7 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
         if items_in_all is not None:
             # the lists, the scratch and the launch are those of the total, whatever the lengths: what is left over are items
             # without rows; the kernel's last part merges, no list of merges is needed
-            items += ([0, 0, 0, 0, -1] + [0] * (FLASH_ITEM_INTS - 5)) * (items_in_all - len(items) // FLASH_ITEM_INTS)
+            items += _NO_ROWS * (items_in_all - len(items) // FLASH_ITEM_INTS)
             n_parts, part_rows, merge = int(items_in_all), max(q_lens[r] for r in rest) * G, []
         plan[f"fa{gi}_items"] = items
         plan[f"fa{gi}_merge"] = merge
@@ -1271,7 +1337,7 @@ def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype
         out[geo] = parts
         if (ctx_lens and parts == 1 and DECODE_ATTENTION_MMA and dtype == torch.bfloat16 and D == 128 and Hq // Hkv <= 16
                 and geometry_planes(geo) >= 2):
-            keys = [attended_keys(1, c, window) for c in ctx_lens]
+            keys = attended_keys([1] * len(ctx_lens), ctx_lens, window)
             wide = DECODE_ATTENTION_MMA_WIDE and num_reqs * Hkv <= TC_TARGET_CTAS          # CTAs of 8 warps
             out[geo] = parts_for_lengths(geo, keys, -(-max(keys) // (2 if wide else 1))) or parts
     return out

@@ -108,7 +108,7 @@ def test_parts_by_length_cover_every_key_in_a_fixed_number_of_items(seed):
     items = _items(plan, "fa0_items")
     assert len(items) == total and plan["fa0_info"] == [total, geo[0] // geo[1], 1, geo[0] // geo[1], 0] and plan["fa0_merge"] == []
     of = {r: [i for i in items if i[8] and i[0] == r] for r in range(R)}
-    parts = ops.parts_by_length([ops.attended_keys(1, c, geo[3]) for c in ctx], total)
+    parts = ops.parts_by_length(ops.attended_keys([1] * R, ctx, geo[3]), total)
     used = [i[4] for i in items if i[4] >= 0]
     assert len(set(used)) == len(used) and max(used, default=0) < total
     for r, mine in of.items():
@@ -146,3 +146,51 @@ def test_latent_attention_shares_an_sm_with_no_other_tensor_memory():
         smem = int(ops.lib().qe_latent_attention_tc_smem(D, ctypes.byref(alone)))
         assert alone.value <= smem <= 225 * 1024
         assert smem + 1024 + 60 * 1024 + 1024 > 228 * 1024, D
+
+
+def test_contexts_are_dealt_out_once_and_not_at_all_where_sums_tell(monkeypatch):
+    """A decode step's plan is on the host's path: a batch of equal or nearly equal contexts is told by its sum and by counting the
+    parts that it would need, and one that is cut by length is dealt out once, not by ``decode_splits`` and by the plan again."""
+    geo, bf = (16, 8, 128, 0), torch.bfloat16
+    calls = []
+    real = ops.parts_by_length
+    monkeypatch.setattr(ops, "parts_by_length", lambda *a: calls.append(1) or real(*a))
+
+    def step(ctx):
+        calls.clear()
+        splits = ops.decode_splits(len(ctx), 2048, (geo,), bf, ctx)
+        ops.plan_attention([1] * len(ctx), ctx, 16, (geo,), bf, uniform_splits=splits)
+        return splits[geo]
+    for R in (15, 28, 36, 48, 64, 73):
+        assert step([1000] * R) == 1 and not calls
+        assert step([960 + 16 * (i % 6) for i in range(R)]) == 1 and not calls
+    for ragged in ([150 + 70 * i for i in range(28)], [150 + 130 * i for i in range(15)], [120 + 28 * i for i in range(64)]):
+        assert type(step(ragged)) is ops.TotalParts and len(calls) == 1
+    calls.clear()
+    ops.plan_attention([512] + [1] * 15, [0] + [150 + 130 * i for i in range(15)], 16, (geo,), bf)
+    assert len(calls) == 1
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_a_step_of_decoded_tokens_alone_is_planned_as_the_general_path_does(seed):
+    """The same requests beside one that brings two tokens take the general path: whole contexts, equal parts, parts by length."""
+    rng = random.Random(400 + seed)
+    geo = ((16, 8, 128, 0), (32, 8, 128, 0), (16, 8, 128, 700, True), (6, 2, 48, 0))[seed % 4]
+    R = rng.randint(1, 40)
+    ctx = [rng.choice([0, 255, 256, 1000, rng.randint(1, 5000)]) for _ in range(R)]
+    for parts in (1, 2, 3, 8, ops.TotalParts(2 * R)):
+        one, both = parts, parts
+        if isinstance(parts, ops.TotalParts):
+            both = ops.TotalParts(parts + 1)
+            both.shares = ops.parts_by_length(ops.attended_keys([1] * R, ctx, geo[3]), parts) + [1]
+        got = ops.plan_attention([1] * R, ctx, 16, (geo,), torch.bfloat16, uniform_splits={geo: one})
+        want = ops.plan_attention([1] * R + [2], ctx + [0], 16, (geo,), torch.bfloat16, uniform_splits={geo: both})
+        rows = lambda plan, key, n: [plan[key][i:i + n] for i in range(0, len(plan[key]), n)]
+        held = lambda items: [i for i in items if i[8]]                 # (the items that are left over have no tokens)
+        assert held(rows(got, "fa0_items", 12)) == [i for i in held(rows(want, "fa0_items", 12)) if i[0] != R]
+        assert rows(got, "fa0_merge", 4) == [m for m in rows(want, "fa0_merge", 4) if m[0] != R]
+        assert len(got["fa0_items"]) // 12 == (parts if isinstance(parts, ops.TotalParts) else parts * R)
+        assert got["tiles"] == want["tiles"][:-2]
+        G = geo[0] // geo[1]
+        n_parts = int(parts) if isinstance(parts, ops.TotalParts) else parts * R if parts > 1 else 0
+        assert got["fa0_info"] == [n_parts, G if n_parts else 1, 1, G, parts if parts in (2, 8) and not isinstance(parts, ops.TotalParts) else 0]
