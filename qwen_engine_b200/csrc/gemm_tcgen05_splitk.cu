@@ -253,8 +253,10 @@ static int launch_splitk_rows(const void* x, const void* w, void* out, int M, in
 // shares of K are short and which find room less easily the more they are, and more tokens: 128 rows, a CTA per SM.
 template <int S>
 static int launch_splitk(const void* x, const void* w, void* out, int M, int N, int K, int mode, cudaStream_t stream, int act) {
-  if (S < 8 && M <= 16) return launch_splitk_rows<S, 64, 16, 4>(x, w, out, M, N, K, mode, stream, act);
-  if (S < 8 && M <= 32) return launch_splitk_rows<S, 64, 32, 4>(x, w, out, M, N, K, mode, stream, act);
+  if constexpr (S < 8) {
+    if (M <= 16) return launch_splitk_rows<S, 64, 16, 4>(x, w, out, M, N, K, mode, stream, act);
+    if (M <= 32) return launch_splitk_rows<S, 64, 32, 4>(x, w, out, M, N, K, mode, stream, act);
+  }
   return launch_splitk_rows<S, 128, 64, 3>(x, w, out, M, N, K, mode, stream, act);
 }
 

@@ -1,5 +1,5 @@
-// out[M, N] = x[M, K] · w[N, K]^T in bfloat16 for up to 64 rows, and act(x · gate^T) * (x · up^T) over stacked weights, where
-// the weight rows are many but no multiple of what the other kernels spread evenly: 64 weight rows a CTA.
+// out[M, N] = x[M, K] · w[N, K]^T in bfloat16 for up to 32 rows, and act(x · gate^T) * (x · up^T) over stacked weights for up to
+// 64, where the weight rows are many but no multiple of what the other kernels spread evenly: 64 weight rows a CTA.
 //
 // What bounds it: the weights' way from memory.  gemm_tcgen05_swap.cu gives 128 weight rows to a CTA that fills an SM's
 // shared memory, so 19 456 rows (Qwen3-4B's gate and up) are 152 CTAs, four more than the SMs, and take two rounds, and
@@ -210,15 +210,18 @@ extern "C" void qe_gemm_tc_stream_clear_status() {
 }
 
 // (the ring's stages: three CTAs per SM up to 32 tokens, two beyond)
-#define SR_DISPATCH(T, GLU) do { \
-    if (M <= 16) return launch_stream<T, 16, 3, GLU>(x, w, out, M, N, K, act, stream); \
-    if (M <= 32) return launch_stream<T, 32, 3, GLU>(x, w, out, M, N, K, act, stream); \
-    return launch_stream<T, 64, 3, GLU>(x, w, out, M, N, K, act, stream); } while (0)
+template <typename TOut, bool GLU>
+static int launch_stream_rows(const void* x, const void* w, void* out, int M, int N, int K, int act, cudaStream_t stream) {
+  if (M <= 16) return launch_stream<TOut, 16, 3, GLU>(x, w, out, M, N, K, act, stream);
+  if (M <= 32) return launch_stream<TOut, 32, 3, GLU>(x, w, out, M, N, K, act, stream);
+  if constexpr (GLU) return launch_stream<TOut, 64, 3, GLU>(x, w, out, M, N, K, act, stream);
+  QE_REFUSE("linear_tcgen05_stream: M = %d is above 32", M);
+}
 
-// The forms of qe_linear_tcgen05_swap (which has checked the operands) with 64 weight rows a CTA, 1 <= M <= 64.  glu: N outputs
-// over w [2 N, K], act as glu_fast takes it, out bfloat16; else act as act_for does.
+// The forms of qe_linear_tcgen05_swap (which has checked the operands) with 64 weight rows a CTA, 1 <= M <= 32.  glu: N outputs
+// over w [2 N, K], M <= 64, act as glu_fast takes it, out bfloat16; else act as act_for does.
 int qe_gemm_tc_stream(const void* x, const void* w, void* out, int M, int N, int K, int out_f32, int act, bool glu, cudaStream_t stream) {
-  if (glu) SR_DISPATCH(__nv_bfloat16, true);
-  if (out_f32) SR_DISPATCH(float, false);
-  SR_DISPATCH(__nv_bfloat16, false);
+  if (glu) return launch_stream_rows<__nv_bfloat16, true>(x, w, out, M, N, K, act, stream);
+  if (out_f32) return launch_stream_rows<float, false>(x, w, out, M, N, K, act, stream);
+  return launch_stream_rows<__nv_bfloat16, false>(x, w, out, M, N, K, act, stream);
 }

@@ -183,8 +183,8 @@ extern "C" void qe_gemm_tc_swap_clear_status() {
 
 int qe_gemm_tc_stream(const void* x, const void* w, void* out, int M, int N, int K, int out_f32, int act, bool glu, cudaStream_t stream);
 
-// form 0: 128 weight rows a CTA (this file), 1 <= M <= 256.  form 1: 64 weight rows a CTA (gemm_tcgen05_stream.cu), M <= 64.  form
-// 2: the same over stacked weights w [2 N, K], out[M, N] = glu(x · w[:N]^T, x · w[N:]^T) in bfloat16, glu_act as glu_fast takes it.
+// form 0: 128 weight rows a CTA (this file), 1 <= M <= 256.  form 1: 64 weight rows a CTA (gemm_tcgen05_stream.cu), M <= 32.  form
+// 2: the same over stacked weights w [2 N, K], M <= 64, out[M, N] = glu(x · w[:N]^T, x · w[N:]^T) in bfloat16, glu_act as glu_fast takes it.
 // Returns 0 when run, 1 when refused (qe_last_error says why), 2 on a launch error.
 extern "C" int qe_linear_tcgen05_swap(const void* x, const void* w, void* out, int M, int N, int K, int out_mode, int form, int glu_act,
                                       cudaStream_t stream) {
@@ -192,7 +192,8 @@ extern "C" int qe_linear_tcgen05_swap(const void* x, const void* w, void* out, i
   if (act < 0 || act > QE_ACT_MAX) QE_REFUSE("linear_tcgen05_swap: unknown activation %d", act);
   if (form < 0 || form > 2 || (form == 2 && out_mode)) QE_REFUSE("linear_tcgen05_swap: form %d, output mode %d", form, out_mode);
   if (M <= 0 || N <= 0) return 0;
-  if (M > (form ? 64 : 256)) QE_REFUSE("linear_tcgen05_swap: M = %d is above %d", M, form ? 64 : 256);
+  const int most = form == 0 ? 256 : form == 1 ? 32 : 64;
+  if (M > most) QE_REFUSE("linear_tcgen05_swap: M = %d is above %d", M, most);
   if (K <= 0 || K % 8) QE_REFUSE("linear_tcgen05_swap: K = %d is not a positive multiple of 8", K);
   // (the forms of 64 rows store element by element)
   if (((uintptr_t)x | (uintptr_t)w | (form ? 0 : (uintptr_t)out)) & 15) QE_REFUSE("linear_tcgen05_swap: operands must be 16-byte aligned");

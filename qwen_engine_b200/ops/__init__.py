@@ -62,7 +62,7 @@ DECODE_ATTENTION_MMA_BESIDE_TC = True   # also for the decoded tokens of a step 
 SHIFTS_IN_ONE_LAUNCH = True          # a mixer that mixes its heads' weights: the shifts of the values' kv head as one launch where the step has no long portion
 DECODE_ATTENTION_MMA_WIDE = True    # steps with at most as many attention CTAs as SMs: CTAs of 8 warps, one per SM (and contexts split for 148 CTAs, not 296)
 DECODE_PARTS_BY_LENGTH = True          # decode steps of many requests with contexts of unequal lengths: parts in proportion to them
-DECODE_PART_MIN_KEYS = 256             # ... none shorter than this
+DECODE_PART_MIN_KEYS = 256             # ... of at least this many on average
 DECODE_PART_COST_KEYS = 96             # what the merge of a cut context costs, in keys of a CTA of 4 warps
 LATENT_DECODE = True                 # decoded tokens over a latent cache (one plane, one kv head): the kernel whose warps stream key groups of their own
 LATENT_DECODE_MIN_PART = 128         # keys of a part at least where a step's contexts are cut for that kernel
@@ -1092,13 +1092,15 @@ def attended_keys(q_lens: list[int], ctx_lens: list[int], window: int) -> list[i
 
 def parts_by_length(keys: list[int], total: int) -> list[int]:
     """How many parts each of the requests with so many keys is cut into, at most ``total`` in all (at least one each): the
-    next part goes to the request whose parts are longest, until those are short."""
+    next part goes to the request whose parts are longest, until another would leave it parts of less than
+    ``DECODE_PART_MIN_KEYS`` on average (the kernel rounds a part up to its groups of 16 keys, so a request's last part holds
+    what is left over, or nothing)."""
     parts = [1] * len(keys)
     longest = [(-n, i) for i, n in enumerate(keys)]
     heapq.heapify(longest)
     for _ in range(total - len(keys)):
-        n, i = longest[0]
-        if -n < 2 * DECODE_PART_MIN_KEYS and -keys[i] / (parts[i] + 1) > -DECODE_PART_MIN_KEYS:
+        i = longest[0][1]
+        if keys[i] / (parts[i] + 1) < DECODE_PART_MIN_KEYS:
             break
         parts[i] += 1
         heapq.heapreplace(longest, (-keys[i] / parts[i], i))

@@ -65,3 +65,13 @@ def test_very_many_weight_rows_go_64_to_a_cta():
     assert all(glu(M, "4b") and glu(M, "1.7b") for M in (1, 8, 16, 17, 64)) and not glu(65, "4b")
     assert not glu(8, "0.6b") and not glu(16, "0.6b") and glu(17, "0.6b") and glu(64, "0.6b")
     assert not ops.swiglu_stream_applies(28, 3072, 4096, BF), "K too long for a CTA alone"
+
+
+def test_rows_beyond_what_a_form_serves_are_refused():
+    """64 weight rows a CTA: up to 32 rows as they are, up to 64 with the activation (refused before anything is launched)."""
+    import ctypes
+    at = ctypes.c_void_p(1 << 20)
+    call = lambda M, form: ops.lib().qe_linear_tcgen05_swap(at, at, at, M, 128, 64, 0, form, 0, ctypes.c_void_p(0))
+    for M, form, most in ((33, 1, b"32"), (64, 1, b"32"), (65, 2, b"64"), (257, 0, b"256")):
+        assert call(M, form) == 1 and b"above " + most in ops.lib().qe_last_error()
+    assert call(8, 3) == 1 and ops.STREAM_MAX_M == 32 and ops.STREAM_GLU_MAX_M == 64
