@@ -63,7 +63,9 @@ SHIFTS_IN_ONE_LAUNCH = True          # a mixer that mixes its heads' weights: th
 DECODE_ATTENTION_MMA_WIDE = True    # steps with at most as many attention CTAs as SMs: CTAs of 8 warps, one per SM (and contexts split for 148 CTAs, not 296)
 DECODE_PARTS_BY_LENGTH = True          # decode steps of many requests with contexts of unequal lengths: parts in proportion to them
 DECODE_PART_MIN_KEYS = 256             # ... of at least this many on average
-DECODE_PART_COST_KEYS = 96             # what the merge of a cut context costs, in keys of a CTA of 4 warps
+DECODE_PART_COST_KEYS = 48             # what cutting contexts costs for each row of an item, in keys of a CTA of 4 warps
+DECODE_PARTS_SECOND_ROUND = 1.4        # rounds of whole contexts from which a second round of parts costs no more than that
+DECODE_PARTS_BESIDE_TC_MAX = 4         # beside prompt portions: parts per request above which contexts stay cut into equally many
 LATENT_DECODE = True                 # decoded tokens over a latent cache (one plane, one kv head): the kernel whose warps stream key groups of their own
 LATENT_DECODE_MIN_PART = 128         # keys of a part at least where a step's contexts are cut for that kernel
 DECODE_PREFETCH_KV_MB = 12          # that kernel asks L2 for the next layer's keys and values when a layer's are at most this many MB (0: never).  Measured (0.6B, context 1 024, asked for before the kernel's dependency wait): 4.4 MB (one request) 0.698 -> 0.690 ms a step, 8.8 MB 0.777 -> 0.765, 17.6 MB equal, 35 MB (eight) 0.915 -> 0.957
@@ -1107,21 +1109,30 @@ def parts_by_length(keys: list[int], total: int) -> list[int]:
     return parts
 
 
-def parts_for_lengths(geo, keys: list[int], one_each: int) -> Optional[TotalParts]:
-    """The work items to deal out by length among requests with so many keys where that is faster than contexts of which the
-    longest part has ``one_each`` keys (in keys of a CTA of 4 warps, two per SM); None where it is not.
+def parts_for_lengths(geo, keys: list[int], one_each: int, rows: int) -> Optional[TotalParts]:
+    """The work items (of ``rows`` rows) to deal out by length among requests with so many keys where that is faster than contexts
+    of which the longest part has ``one_each`` keys (in keys of a CTA of 4 warps, two per SM); None where it is not.
 
-    The longest part sets the time, or the keys of all where the parts are even.  Measured on a B200 (kv heads 8, a chain of
-    launches): 28 requests of 130 to 2 045 keys 37.2 us whole, 27.5 in 37 parts (one wave), 31.8 in 55; 15 such 24.8 whole (8
-    warps each), 16.0 in 37 parts; 64 of 985 on average 56.7 whole, 51.6 in 74 (two waves); one of 16 384 beside 15 of 200
-    199 whole, 22.6 in 37.  Contexts of equal lengths gain nothing (16 of 1 400: 20.9 whole, 22.1 in 37) and stay whole."""
+    The longest part sets the time, or the keys of all where the parts are even; a part's accumulators go through memory, row by
+    row.  Measured on a B200 (kv heads 8, two rows, a chain of launches): 28 requests of 130 to 2 045 keys 37.2 us whole, 27.5 in 37
+    parts (one round of CTAs), 31.8 in 55; 15 such 24.8 whole (8 warps each), 16.0 in 37 parts; 64 of 985 on average 56.7 whole, 51.6
+    in 74 (two rounds); one of 16 384 beside 15 of 200 199 whole, 22.6 in 37.  Contexts of equal lengths gain nothing (16 of
+    1 400: 20.9 whole, 22.1 in 37) and stay whole; with more rows a part costs more (10 of 1 000 in 30 parts: two rows 13.6 -> 13.1, four
+    14.1 -> 14.9, eight 14.6 -> 18.0).  Where whole contexts fill one round or little more, a second round of parts costs its own start
+    and drains what was even: 37 of 800 to 1 200 29.0 -> 34.6 us with two rows, 29.7 -> 38.9 with four, 40 of 130 to 1 760 36.4 -> 37.2
+    and 36.5 -> 40.9.  (Over 728 batches of 1 to 8 rows and 1 to 8 kv heads, equal, ragged, with one or a few long contexts, nothing that
+    these lines cut is more than 1 % slower for it.)"""
     slots = FLASH_TARGET_CTAS // (geo[1] * value_blocks(geo))
-    total = slots if len(keys) < slots else 2 * slots
-    if not DECODE_PARTS_BY_LENGTH or slots < 1 or len(keys) >= total or total * geo[1] * value_blocks(geo) > _MERGE_COUNTERS:
+    n = len(keys)
+    total = slots if n < slots else 2 * slots
+    if not DECODE_PARTS_BY_LENGTH or slots < 1 or n >= total or total * geo[1] * value_blocks(geo) > _MERGE_COUNTERS:
         return None
     even = sum(keys) / slots
+    cost = DECODE_PART_COST_KEYS * rows
+    if slots <= n < DECODE_PARTS_SECOND_ROUND * slots:
+        cost = 100 + 100 * rows + 0.4 * even
     # below this many keys the longest part has to stay; sums and counts tell most batches apart before anything is dealt out
-    limit = max(one_each, even) - DECODE_PART_COST_KEYS
+    limit = max(one_each, even) - cost
     most = math.ceil(limit) - 1
     if even >= limit or most < 1 or sum([-(-n // most) for n in keys]) > total:
         return None
@@ -1226,8 +1237,11 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
         elif (rest and len(rest) < len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_BESIDE_TC and D == 128
               and geometry_planes(geo) >= 2 and max(q_lens[r] for r in rest) * G <= 16):
             at_most = max(1, FLASH_TARGET_CTAS // base)
-            keys = attended_keys([q_lens[r] for r in rest], [ctx_lens[r] for r in rest], window)
-            items_in_all = parts_for_lengths(geo, keys, max(-(-k // min(-(-k // FLASH_SPLIT), at_most)) for k in keys))
+            if at_most <= DECODE_PARTS_BESIDE_TC_MAX:
+                # (above: 7 contexts of 350 keys and one of 3 500 beside a portion of 300, 40.6 -> 42.6 us)
+                keys = attended_keys([q_lens[r] for r in rest], [ctx_lens[r] for r in rest], window)
+                items_in_all = parts_for_lengths(geo, keys, max(-(-k // min(-(-k // FLASH_SPLIT), at_most)) for k in keys),
+                                                 max(q_lens[r] for r in rest) * G)
         if items_in_all is not None:
             dealt = items_in_all.shares
             if dealt is None:
@@ -1341,7 +1355,7 @@ def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype
                 and geometry_planes(geo) >= 2):
             keys = attended_keys([1] * len(ctx_lens), ctx_lens, window)
             wide = DECODE_ATTENTION_MMA_WIDE and num_reqs * Hkv <= TC_TARGET_CTAS          # CTAs of 8 warps
-            out[geo] = parts_for_lengths(geo, keys, -(-max(keys) // (2 if wide else 1))) or parts
+            out[geo] = parts_for_lengths(geo, keys, -(-max(keys) // (2 if wide else 1)), geo[0] // geo[1]) or parts
     return out
 
 

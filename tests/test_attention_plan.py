@@ -118,6 +118,13 @@ def test_parts_by_length_cover_every_key_in_a_fixed_number_of_items(seed):
         else:
             mine.sort(key=lambda i: i[6])
             assert [i[4:7] for i in mine] == [[mine[0][4] + s, len(mine), s] for s in range(len(mine))]
+            # the keys of a part as the kernel works them out: equal shares rounded up to its groups of 16 keys, from the first key
+            # tile that the window reaches on; together they are every key that the token attends to, each once
+            lo = max(0, ctx[r] - geo[3] + 1) // ops.FLASH_BN * ops.FLASH_BN if geo[3] else 0
+            per = -(-(-(-(ctx[r] + 1 - lo) // len(mine))) // 16) * 16
+            spans = [(lo + s * per, min(ctx[r] + 1, lo + (s + 1) * per)) for s in range(len(mine))]
+            keys = [k for a, b in spans for k in range(a, b)]
+            assert keys == list(range(lo, ctx[r] + 1)) and keys[0] <= max(0, ctx[r] - geo[3] + 1 if geo[3] else 0)
     empty = [i for i in items if not i[8]]
     assert len(empty) == total - sum(parts) and all(i == [0, 0, 0, 0, -1] + [0] * 7 for i in empty)
 
@@ -194,3 +201,32 @@ def test_a_step_of_decoded_tokens_alone_is_planned_as_the_general_path_does(seed
         G = geo[0] // geo[1]
         n_parts = int(parts) if isinstance(parts, ops.TotalParts) else parts * R if parts > 1 else 0
         assert got["fa0_info"] == [n_parts, G if n_parts else 1, 1, G, parts if parts in (2, 8) and not isinstance(parts, ops.TotalParts) else 0]
+
+
+@pytest.mark.parametrize("heads,kv_heads,ctx", [
+    (16, 8, [800 + 11 * i for i in range(37)]),             # one round of whole contexts: 29.0 us whole, 34.6 cut
+    (32, 8, [800 + 11 * i for i in range(37)]),             # 29.7, 38.9
+    (32, 8, [130 + 42 * i for i in range(39)]),             # 26.9, 31.7
+    (32, 8, [175 + 1225 * (i % 2) for i in range(48)]),     # 39.3, 42.4
+    (32, 4, [560 + 4 * i for i in range(74)]),              # 21.8, 38.0
+    (16, 1, [560 + i for i in range(296)]),                 # 25.2, 52.2
+    (64, 8, [1000] * 10),                                   # eight rows an item: 14.6, 18.0
+    (64, 8, [150] * 10 + [900] * 3),                        # 12.0, 15.8
+    (32, 8, [1000] * 12),                                   # 14.6, 15.7
+])
+def test_contexts_stay_whole_where_cutting_them_costs_more(heads, kv_heads, ctx):
+    geo, bf = (heads, kv_heads, 128, 0), torch.bfloat16
+    splits = ops.decode_splits(len(ctx), -(-max(ctx) // 1024) * 1024, (geo,), bf, ctx)[geo]
+    assert type(splits) is int
+    beside = ops.plan_attention([512] + [1] * len(ctx), [0] + ctx, 16, (geo,), bf)
+    whole = ops.FLASH_TARGET_CTAS // (len(ctx) * kv_heads) <= 1
+    assert not whole or beside["fa0_info"][0] == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,ctx", [
+    (16, 8, [150 + 70 * i for i in range(28)]), (64, 8, [200] * 16 + [4000]), (32, 8, [150 + 130 * i for i in range(15)]),
+    (16, 8, [200] * 36 + [8192]), (32, 8, [350] * 55 + [3500]), (16, 4, [150 + 50 * i for i in range(111)]), (16, 1, [200] * 99 + [8192]),
+])
+def test_contexts_are_cut_where_one_of_them_sets_the_time(heads, kv_heads, ctx):
+    geo, bf = (heads, kv_heads, 128, 0), torch.bfloat16
+    assert type(ops.decode_splits(len(ctx), -(-max(ctx) // 1024) * 1024, (geo,), bf, ctx)[geo]) is ops.TotalParts
