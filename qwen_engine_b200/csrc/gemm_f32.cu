@@ -1,6 +1,6 @@
 // The float32 product (see gemm_f32.cuh): every multiply-add is a float32 fma, two at a time (`fma.rn.f32x2`).
 //
-// Order of a sum, whatever M is: K is cut into S equal chunks (a function of N and K alone), a chunk into runs of 16 that
+// Order of a sum, whatever M is: K is cut into S equal chunks of whole runs (a function of N and K alone), a chunk into runs of 16 that
 // are dealt to four groups in turn; a group's k are summed as two chains, the even and the odd ones, and even + odd, the
 // groups and the chunks are added in order.  So a row's bits do not depend on
 // what else is in the batch, and the chains are 8 S times shorter than one over all of K.
@@ -11,7 +11,7 @@
 //    are conflict-free) by 16-byte cp.async, several k-blocks ahead; with at most 16 rows the weights' first blocks are
 //    asked for before the wait for the kernel before;
 //  - a thread keeps TM x TN pairs of sums and reads 4 k of a row in one load: the pair (k, k + 1) is the register pair that
-//    the two-wide fma takes, so nothing is packed or duplicated; up to 8 x 8 sums, since a 16-byte load from shared memory
+//    the two-wide fma takes, so nothing is packed or duplicated; up to 8 x 4 sums, since a 16-byte load from shared memory
 //    costs four of its cycles even where lanes read the same word;
 //  - up to 16 rows the four groups are warps of their own, so that a tile has enough of them to hide its loads (a block is 64
 //    k, a run of each); beyond, a thread takes one group after the other (a block is two runs of a group);
@@ -53,7 +53,8 @@ struct GfShape {
   static_assert((size_t)(SLICED ? GF_GROUPS : 1) * BM * GF_BN * sizeof(float) <= SMEM, "the groups' partial tiles take the stages' place");
 };
 
-template <int BM, int TM, int TN, int STAGES>
+// TAIL: runs behind the share's end are neither loaded nor summed (a group's blocks hold two runs each).
+template <int BM, int TM, int TN, int STAGES, bool TAIL>
 __global__ void __launch_bounds__(GfShape<BM, TM, TN, STAGES>::THREADS, GfShape<BM, TM, TN, STAGES>::CTAS)
 gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out,
                 int M, int N, int K, int chunk, int splits, int act, int vec) {
@@ -66,11 +67,13 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   // blocks to load: of a run of each group; or, where a thread takes the groups in turn, `turn` of two runs for each
   const int rounds = (k_end - k_begin + GF_GROUPS * GF_RUN - 1) / (GF_GROUPS * GF_RUN);
   const int turn = (rounds + 1) / 2;
-  const int blocks = S::SLICED ? rounds : turn * GF_GROUPS;
+  const int groups = TAIL && rounds == 1 ? (k_end - k_begin + GF_RUN - 1) / GF_RUN : GF_GROUPS;     // that have any k
+  const int blocks = S::SLICED ? rounds : turn * groups;
   constexpr int LD = S::LD, WORDS = S::BK / 4;                      // 16-byte words of a row's k-block
   static_assert(S::THREADS % WORDS == 0, "a thread's words are the same one of every row");
   const int word = threadIdx.x % WORDS, row = threadIdx.x / WORDS;
   const int word_k = S::SLICED ? word * 4 : word / (GF_RUN / 4) * (GF_GROUPS * GF_RUN) + word % (GF_RUN / 4) * 4;
+  const int k_in_run = word_k % GF_RUN;
   auto k_of = [&](int b) {                              // the k of this thread's word of block b
     if (S::SLICED) return k_begin + b * S::BK + word_k;
     const int group = b / turn;
@@ -79,6 +82,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   auto load_w = [&](int b) {
     float* ws = gf_smem + (b % STAGES) * S::STAGE + word * 4;
     const int k = k_of(b);
+    if (TAIL && k - k_in_run >= k_end) return;
 #pragma unroll
     for (int r = row; r < GF_BN; r += S::THREADS / WORDS) {
       const bool ok = n0 + r < N && k < k_end;
@@ -88,6 +92,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   auto load_x = [&](int b) {
     float* xs = gf_smem + (b % STAGES) * S::STAGE + GF_BN * LD + word * 4;
     const int k = k_of(b);
+    if (TAIL && k - k_in_run >= k_end) return;
 #pragma unroll
     for (int r = row; r < BM; r += S::THREADS / WORDS) {
       const bool ok = m0 + r < M && k < k_end;
@@ -125,6 +130,8 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
 
   const int offset = S::SLICED ? group * GF_RUN : 0;
   int left = turn;                                      // blocks of the group in turn
+  int k_run = k_begin + offset;                         // where this block's (first) run starts
+  int k_next = k_begin + GF_RUN;                        // ... and the first of the group after the one in turn
 #pragma unroll 1
   for (int b = 0; b < blocks; ++b) {
     asm volatile("cp.async.wait_group %0;\n" :: "n"(STAGES - 2) : "memory");
@@ -134,23 +141,30 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     const float* ws = gf_smem + (b % STAGES) * S::STAGE + tn * LD + offset;
     const float* xs = gf_smem + (b % STAGES) * S::STAGE + (GF_BN + tm) * LD + offset;
 #pragma unroll
-    for (int k = 0; k < (S::SLICED ? GF_RUN : S::BK); k += 4) {
-      ulonglong2 a[TM], c[TN];
+    for (int run = 0; run < S::BK / (S::SLICED ? GF_GROUPS * GF_RUN : GF_RUN); ++run) {
+      if (TAIL && k_run + run * (GF_GROUPS * GF_RUN) >= k_end) break;     // uniform within the group
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * S::MT * LD + k);
+      for (int k = run * GF_RUN; k < (run + 1) * GF_RUN; k += 4) {
+        ulonglong2 a[TM], c[TN];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) c[j] = *reinterpret_cast<const ulonglong2*>(ws + j * S::NT * LD + k);
+        for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xs + i * S::MT * LD + k);
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+        for (int j = 0; j < TN; ++j) c[j] = *reinterpret_cast<const ulonglong2*>(ws + j * S::NT * LD + k);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) gf_fma2(acc[i][j], a[i].x, c[j].x);
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+          for (int j = 0; j < TN; ++j) gf_fma2(acc[i][j], a[i].x, c[j].x);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) gf_fma2(acc[i][j], a[i].y, c[j].y);
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) gf_fma2(acc[i][j], a[i].y, c[j].y);
+      }
     }
+    k_run += S::BK / GF_RUN * (S::SLICED ? GF_RUN : GF_GROUPS * GF_RUN);
     if (!S::SLICED && --left == 0) {
       left = turn;
+      k_run = k_next;
+      k_next += GF_RUN;
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -209,18 +223,18 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   if (splits > 1) cluster_sync_all();                   // the other CTAs read this one's shared memory
 }
 
-template <int BM, int TM, int TN, int STAGES>
+template <int BM, int TM, int TN, int STAGES, bool TAIL = false>
 static int gf_launch(const float* x, const float* w, float* out, int M, int N, int K, int chunk, int splits, int act, cudaStream_t stream) {
   using S = GfShape<BM, TM, TN, STAGES>;
   static const cudaError_t configured =
-      cudaFuncSetAttribute(gemm_f32_kernel<BM, TM, TN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+      cudaFuncSetAttribute(gemm_f32_kernel<BM, TM, TN, STAGES, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
   if (configured != cudaSuccess) QE_REFUSE("linear: shared memory %d: %s", (int)S::SMEM, cudaGetErrorString(configured));
   const dim3 grid((N + GF_BN - 1) / GF_BN * splits, (M + BM - 1) / BM);
   const int vec = N % 4 == 0 && (uintptr_t)out % 16 == 0;
   if (splits > 1)
-    qe_launch_cluster(gemm_f32_kernel<BM, TM, TN, STAGES>, grid, dim3(S::THREADS), S::SMEM, stream, (unsigned)splits, x, w, out, M, N, K, chunk, splits, act, vec);
+    qe_launch_cluster(gemm_f32_kernel<BM, TM, TN, STAGES, TAIL>, grid, dim3(S::THREADS), S::SMEM, stream, (unsigned)splits, x, w, out, M, N, K, chunk, splits, act, vec);
   else
-    qe_launch(gemm_f32_kernel<BM, TM, TN, STAGES>, grid, dim3(S::THREADS), S::SMEM, stream, x, w, out, M, N, K, chunk, splits, act, vec);
+    qe_launch(gemm_f32_kernel<BM, TM, TN, STAGES, TAIL>, grid, dim3(S::THREADS), S::SMEM, stream, x, w, out, M, N, K, chunk, splits, act, vec);
   QE_CHECK_LAUNCH("linear_f32");
   return 0;
 }
@@ -230,13 +244,30 @@ int qe_gemm_f32(const float* x, const float* w, float* out, int M, int N, int K,
   const int tiles = (N + GF_BN - 1) / GF_BN;
   int splits = 1;
   while (splits < 8 && (long)tiles * splits * 2 <= 2 * 148 && K / (2 * splits) >= 128) splits *= 2;
-  const int chunk = ((K + splits - 1) / splits + GF_GROUPS * GF_RUN - 1) / (GF_GROUPS * GF_RUN) * (GF_GROUPS * GF_RUN);
+  const int chunk = ((K + splits - 1) / splits + GF_RUN - 1) / GF_RUN * GF_RUN;
   if (M <= 4) return gf_launch<4, 4, 2, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
   if (M <= 8) return gf_launch<8, 8, 2, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
   if (M <= 16) return gf_launch<16, 8, 4, 3>(x, w, out, M, N, K, chunk, splits, act, stream);
+  // One run of each group at most: the tiles with two runs a block are mostly padding.  The groups' own warps do better up to some
+  // rounds of CTAs, then 48 rows a tile (1 024 x 64 at 256 rows 8.5 -> 3.4 us, at 2 048 20.4 -> 14.5; the kernel of gemm_generic.cu
+  // 6.3 and 16.3).
+  if (K <= GF_GROUPS * GF_RUN) {
+    if ((long)M * N <= 1 << 20 && M <= 1 << 16) return gf_launch<16, 8, 4, 3>(x, w, out, M, N, K, chunk, splits, act, stream);
+    if (M <= 48 * 65535) return gf_launch<48, 6, 4, 4, true>(x, w, out, M, N, K, chunk, splits, act, stream);
+    return gf_launch<64, 8, 4, 4, true>(x, w, out, M, N, K, chunk, splits, act, stream);
+  }
   // rows that the tiles cover, a tile's own cost counted as 8 more
   auto cost = [&](long bm) { return (M + bm - 1) / bm * (bm + 8); };
-  if (M > 4096 || (cost(64) <= cost(48) && cost(64) <= cost(32))) return gf_launch<64, 8, 4, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
-  if (cost(48) <= cost(32)) return gf_launch<48, 6, 4, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
+  const int bm = M > 4096 || (cost(64) <= cost(48) && cost(64) <= cost(32)) ? 64 : cost(48) <= cost(32) ? 48 : 32;
+  // runs behind the share's end are left out where they are a fifth of the work and more (1 024 x 1 056 at 2 048 rows, shares of 144:
+  // 276 -> 209 us, 227 with the kernel of gemm_generic.cu; where they are less, asking costs as much)
+  const int rounds = (chunk + 2 * GF_GROUPS * GF_RUN - 1) / (2 * GF_GROUPS * GF_RUN);
+  if (rounds * 2 * GF_GROUPS * GF_RUN * 4 >= chunk * 5) {
+    if (bm == 64) return gf_launch<64, 8, 4, 4, true>(x, w, out, M, N, K, chunk, splits, act, stream);
+    if (bm == 48) return gf_launch<48, 6, 4, 4, true>(x, w, out, M, N, K, chunk, splits, act, stream);
+    return gf_launch<32, 4, 4, 4, true>(x, w, out, M, N, K, chunk, splits, act, stream);
+  }
+  if (bm == 64) return gf_launch<64, 8, 4, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
+  if (bm == 48) return gf_launch<48, 6, 4, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
   return gf_launch<32, 4, 4, 4>(x, w, out, M, N, K, chunk, splits, act, stream);
 }

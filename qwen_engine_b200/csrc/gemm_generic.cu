@@ -1,5 +1,5 @@
 // out[M, N] = x[M, K] · w[N, K]^T with float32 FMA accumulation, for what the other products refuse: float32 operands that
-// gemm_f32.cu does not take (K no multiple of 4, or an operand off a 16-byte boundary) and bfloat16 shapes that the
+// gemm_f32.cu does not take (K short or no multiple of 4, or an operand off a 16-byte boundary) and bfloat16 shapes that the
 // tensor-core kernels do not take.
 // (reference src/layers/ops/linear.py:101-122: y = x W^T, float32 accumulator.)
 //
@@ -76,7 +76,7 @@ extern "C" int qe_linear_generic(const void* x, const void* w, void* out, int M,
   dim3 grid((N + GG_BN - 1) / GG_BN, (M + GG_BM - 1) / GG_BM);
   if (grid.y > 65535) QE_REFUSE("linear: M %d is too large for the generic kernel", M);
   if (dtype == QE_DTYPE_F32) {
-    if (K % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0)
+    if (K >= GF_MIN_K && K % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0)
       return qe_gemm_f32((const float*)x, (const float*)w, (float*)out, M, N, K, act, stream);
     qe_launch(gemm_generic_kernel<float, float>, grid, dim3(256), 0, stream, (const float*)x, (const float*)w, (float*)out, M, N, K, act);
   } else if (dtype == QE_DTYPE_BF16) {

@@ -358,11 +358,13 @@ def test_linear_row_does_not_depend_on_batch():
         assert torch.equal(one[0], full[r])
 
 
-@pytest.mark.parametrize("N,K", [(1, 4), (63, 36), (130, 1056), (1024, 3072), (4096, 1028), (2500, 100)])
+@pytest.mark.parametrize("N,K", [(1, 4), (63, 36), (130, 44), (130, 48), (4100, 60), (63, 64), (65, 68), (100, 112), (70, 164), (130, 1056),
+                                 (1024, 3072), (4096, 1028), (2500, 100)])
 @pytest.mark.parametrize("Ms", [(1, 4), (5, 8), (9, 16), (17, 32, 33), (48, 49, 64), (65, 141, 257)])
 def test_float32_linear_at_the_edges_of_its_tiles(Ms, N, K):
-    """The 32-bit product at the edges of its row tiles, of 64 weight rows, of runs of 16 k and of the shares of K (1 056
-    in eight shares of 192: the last two have none) against 64 bits.  A sum of K terms in float32, in whatever order, is off by at
+    """The 32-bit product at the edges of its row tiles, of 64 weight rows, of runs of 16 k (short of one, one of some groups only,
+    one run behind K's end) and of the shares of K (1 056 in eight shares of 144: the last has 48), either side of the K from which
+    its kernel serves and of the outputs up to which short K take tiles of 16 rows, against 64 bits.  A sum of K terms in float32, in whatever order, is off by at
     most (K + 8) 2^-24 sum |x w|; a row's bits are the same whatever the number of rows."""
     w = _randn((N, K), torch.float32, 9).to(DEV)
     x = _randn((max(Ms), K), torch.float32, 8).to(DEV)
