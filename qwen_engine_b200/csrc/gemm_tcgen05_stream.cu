@@ -4,12 +4,19 @@
 // What bounds it: the weights' way from memory.  gemm_tcgen05_swap.cu gives 128 weight rows to a CTA that fills an SM's
 // shared memory, so 19 456 rows (Qwen3-4B's gate and up) are 152 CTAs, four more than the SMs, and take two rounds, and
 // 12 288 leave 52 SMs idle.  Here a CTA has 64 rows (the 64-row form of tcgen05.mma) and a ring small enough for two or
-// three CTAs per SM: all of them are on the GPU at once, whatever their number within that, and an SM's loads are as many.
+// three CTAs per SM (three up to 32 rows, two beyond): all of them are on the GPU at once, whatever their number within 444 or
+// 296, and an SM's loads are as many.  What goes beyond that takes another round: 19 456 rows with the activation, 304 CTAs, 18.7 us
+// at 32 rows and 27.4 at 33 (a product and the activation's launch: 32.8 and 33.1).
 // The ring starts with the weights, before the wait for the kernel that writes x.
 //
 // GLU: a CTA's rows are 32 of the gate's and the same 32 of the up projection's (two boxes side by side), and the
 // activation is formed on the float32 sums in the epilogue, rounded once: gate and up never exist in memory, and the
 // activation needs no launch of its own.
+//
+// Precision: tensor memory adds a product in without rounding to nearest, and the error grows with the length of the chain (1e-6 of
+// the result for K = 1 024 in one chain, 4e-6 for 4 096).  Up to 16 rows, where the weight-streaming product gives the k to eight
+// warps at most, every 64 k go to the next of eight accumulators of 16 columns, which are added up in order at the end: chains no
+// longer than there (151 936 x 1 024 1.3e-7, that product 2.2e-7; 16 384 x 4 096 both 4.8e-7).  It costs 0.5 us a round of CTAs.
 //
 // Six warps as in gemm_tcgen05_swap.cu: TMA, MMA, and four that read the accumulator (the 64-row form keeps row r in lane
 // r mod 16 of the quarter r / 16), put it into the ring's memory as [token][row] and store whole runs of a token's outputs.
@@ -41,14 +48,24 @@ struct __align__(1024) SrSmem {
   int abort_flag;
 };
 
-template <typename TOut, int BT, int STAGES, bool GLU>
+// 16 columns of this warp's quarter of the lanes (a lane's row), to be waited for
+__device__ __forceinline__ void sr_load16(uint32_t at, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(at) : "memory");
+}
+
+template <typename TOut, int BT, int STAGES, bool GLU, int ACCS>    // ACCS: accumulators, BT columns each
 __global__ void __launch_bounds__(SR_THREADS)
 gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                            TOut* __restrict__ out, int M, int N, int K, int act) {
   extern __shared__ unsigned char smem_raw[];
   using Smem = SrSmem<BT, STAGES>;
   static_assert(sizeof(float) * BT * SR_BM <= sizeof(__nv_bfloat16) * STAGES * SR_BM * SR_BK, "the sums take the ring's place");
-  constexpr uint32_t TMEM_COLS = BT < 32 ? 32 : BT;
+  constexpr uint32_t TMEM_COLS = BT * ACCS < 32 ? 32 : BT * ACCS;
   constexpr int COLS = GLU ? SR_BM / 2 : SR_BM;       // outputs of a token per CTA
   pdl_launch_dependents();
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -119,7 +136,8 @@ gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         const uint64_t da = make_smem_desc(smem_u32(sm.w[s][h]));
         const uint64_t db = make_smem_desc(smem_u32(sm.x[s][h]));
 #pragma unroll
-        for (int k = 0; k < SR_HALF / 16; ++k) tc_mma_bf16_elect(tmem, da + 2 * k, db + 2 * k, idesc, (kb | h | k) != 0);
+        for (int k = 0; k < SR_HALF / 16; ++k)
+          tc_mma_bf16_elect(tmem + (2 * kb + h) % ACCS * BT, da + 2 * k, db + 2 * k, idesc, 2 * kb + h >= ACCS || k != 0);
       }
       tc_commit_elect(&sm.empty[s]);
     }
@@ -132,17 +150,29 @@ gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     if (ok) {
 #pragma unroll 1
       for (int c0 = 0; c0 < mt; c0 += 16) {
-        uint32_t r[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(tmem + ((uint32_t)(quarter * 32) << 16) + c0) : "memory");
-        tc_wait_ld();
+        constexpr int AT_ONCE = ACCS < 4 ? ACCS : 4;
+        float r[16];
+#pragma unroll
+        for (int a0 = 0; a0 < ACCS; a0 += AT_ONCE) {
+          if (a0 >= 2 * num_kb) break;                  // accumulators that no k reached hold nothing
+          uint32_t u[AT_ONCE][16];
+#pragma unroll
+          for (int a = 0; a < AT_ONCE; ++a) sr_load16(tmem + ((uint32_t)(quarter * 32) << 16) + (a0 + a) * BT + c0, u[a]);
+          tc_wait_ld();
+#pragma unroll
+          for (int a = 0; a < AT_ONCE; ++a)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(u[a][j]));      // (not read before the wait)
+#pragma unroll
+          for (int a = 0; a < AT_ONCE; ++a) {
+            const bool any = a0 + a < 2 * num_kb;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) r[j] = a0 + a == 0 ? __uint_as_float(u[a][j]) : r[j] + (any ? __uint_as_float(u[a][j]) : 0.f);
+          }
+        }
         if (lane < 16) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) sums[(c0 + j) * SR_BM + quarter * 16 + lane] = __uint_as_float(r[j]);
+          for (int j = 0; j < 16; ++j) sums[(c0 + j) * SR_BM + quarter * 16 + lane] = r[j];
         }
       }
     }
@@ -172,7 +202,7 @@ gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
   }
 }
 
-template <typename TOut, int BT, int STAGES, bool GLU>
+template <typename TOut, int BT, int STAGES, bool GLU, int ACCS = 1>
 static int launch_stream(const void* x, const void* w, void* out, int M, int N, int K, int act, cudaStream_t stream) {
   CUtensorMap map_w, map_x;
   {
@@ -188,12 +218,12 @@ static int launch_stream(const void* x, const void* w, void* out, int M, int N, 
     if (!qe_tensor_map_bf16(x, 2, dims, strides, box, &map_x)) return 1;
   }
   const size_t smem = sizeof(SrSmem<BT, STAGES>) + 1024;
-  static_assert(tc_room_for_all(sizeof(SrSmem<BT, STAGES>) + 1024, BT < 32 ? 32 : BT), "tensor memory for every CTA that finds room on an SM");
+  static_assert(tc_room_for_all(sizeof(SrSmem<BT, STAGES>) + 1024, BT * ACCS < 32 ? 32 : BT * ACCS), "tensor memory for every CTA that finds room on an SM");
   static const cudaError_t configured =
-      cudaFuncSetAttribute(gemm_tcgen05_stream_kernel<TOut, BT, STAGES, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(gemm_tcgen05_stream_kernel<TOut, BT, STAGES, GLU, ACCS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (configured != cudaSuccess) QE_REFUSE("linear_tcgen05_stream: shared memory %zu: %s", smem, cudaGetErrorString(configured));
   const int cols = GLU ? SR_BM / 2 : SR_BM;
-  qe_launch(gemm_tcgen05_stream_kernel<TOut, BT, STAGES, GLU>, dim3((unsigned)((N + cols - 1) / cols)), dim3(SR_THREADS), smem, stream,
+  qe_launch(gemm_tcgen05_stream_kernel<TOut, BT, STAGES, GLU, ACCS>, dim3((unsigned)((N + cols - 1) / cols)), dim3(SR_THREADS), smem, stream,
             map_w, map_x, (TOut*)out, M, N, K, act);
   QE_CHECK_LAUNCH("linear_tcgen05_stream");
   return 0;
@@ -212,10 +242,10 @@ extern "C" void qe_gemm_tc_stream_clear_status() {
 // (the ring's stages: three CTAs per SM up to 32 tokens, two beyond)
 template <typename TOut, bool GLU>
 static int launch_stream_rows(const void* x, const void* w, void* out, int M, int N, int K, int act, cudaStream_t stream) {
-  if (M <= 16) return launch_stream<TOut, 16, 3, GLU>(x, w, out, M, N, K, act, stream);
+  if (M <= 16) return launch_stream<TOut, 16, 3, GLU, GLU ? 1 : 8>(x, w, out, M, N, K, act, stream);
   if (M <= 32) return launch_stream<TOut, 32, 3, GLU>(x, w, out, M, N, K, act, stream);
   if constexpr (GLU) return launch_stream<TOut, 64, 3, GLU>(x, w, out, M, N, K, act, stream);
-  QE_REFUSE("linear_tcgen05_stream: M = %d is above 32", M);
+  else QE_REFUSE("linear_tcgen05_stream: M = %d is above 32", M);
 }
 
 // The forms of qe_linear_tcgen05_swap (which has checked the operands) with 64 weight rows a CTA, 1 <= M <= 32.  glu: N outputs

@@ -494,13 +494,14 @@ def stream_applies(M: int, N: int, K: int, dtype: torch.dtype) -> bool:
     x 1 024 at 1, 8, 16 and 28 rows 56 -> 51, 65 -> 53, 79 -> 56 and 64 -> 58 us, x 2 560 128 -> 113, 141 -> 117, 167 -> 120
     and 132 -> 123; 24 576 x 2 048 23.5 -> 16.9 at one row, 29.3 -> 17.6 at 16; 16 384 x 4 096 32.9 -> 24.9.  Up to 8 rows
     it loses where its CTAs are a little more than a round of three per SM (32 768 x 1 024: 15.0 -> 15.5; at 16 rows, where
-    the other kernels re-read x for two tiles of tokens, 21.2 -> 16.0)."""
+    the other kernels re-read x for two tiles of tokens, 21.2 -> 16.0) and where K is short and the weight rows not very many (16 384 x
+    200: 4.7 -> 5.3 at 4 rows)."""
     if not (STREAM and TCGEN05_ENABLED and dtype == torch.bfloat16 and 1 <= M <= STREAM_MAX_M and K % 8 == 0):
         return False
     if M > 16:
         return N >= STREAM_WIDE_MIN_N
     rounds = -(-N // 64) / (3 * TC_TARGET_CTAS)
-    return N >= STREAM_MIN_N and (M > 8 or not 1 < rounds < 1.5)
+    return N >= STREAM_MIN_N and (M > 8 or not (1 < rounds < 1.5 or (K < 512 and rounds < 1)))
 
 
 def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = None) -> None:
@@ -638,7 +639,12 @@ def swiglu_stream_applies(M: int, I: int, K: int, dtype: torch.dtype) -> bool:
     16, 29.7 -> 18.1 at 28; 12 288 x 2 048 11.5 -> 10.6, 13.4 -> 10.7, 13.6 -> 11.2, at 64 rows 15.1 -> 12.5; 6 144 x 1 024
     3.8 -> 5.5 and 5.0 -> 5.7, but 7.1 -> 6.3 at 28 rows and 8.1 -> 7.2 at 64.  A CTA walks all of K (0.27 us for 128 of it), so
     it loses where K is long against the rows (6 144 x 4 096 at 28 rows 13.5 -> 15.9), and up to 8 rows where K is short
-    (16 384 x 1 024 7.1 -> 8.2)."""
+    (16 384 x 1 024 7.1 -> 8.2).  Between the points that drew the lines: 10 240 x 2 560 14.2 -> 11.9 at 8 rows, 16.5 -> 12.2 at 16,
+    8 192 x 2 560 9.5 -> 11.1 and 11.4 -> 11.1, and beyond 16 rows even (11.9 -> 11.7 at 24); 9 728 x 896 up to 8 rows even, at 16
+    7.0 -> 6.0 (not taken).  Beyond 32 rows two CTAs fit an SM instead of three, and more than 296 of them take another round, which
+    is still less than the product and the activation's launch: 19 456 x 2 560 (304 CTAs) 32.8 -> 18.7 at 32 rows, 33.1 -> 27.4 at
+    33, 35.0 -> 29.2 at 64; 24 576 x 4 096 (384) 49.6 -> 35.0, 50.0 -> 42.9, 52.0 -> 45.0; 34 816 x 5 120 (544: more than one round
+    of three too) 63.6 -> 63.2, 64.0 -> 60.3, 66.8 -> 62.8."""
     if not (STREAM and TCGEN05_ENABLED and dtype == torch.bfloat16 and 1 <= M <= STREAM_GLU_MAX_M and K % 8 == 0):
         return False
     few = M <= SWIGLU_SMALL_MAX_M

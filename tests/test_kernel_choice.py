@@ -59,6 +59,7 @@ def test_very_many_weight_rows_go_64_to_a_cta():
     for K in (1024, 2048, 2560):
         assert all(ops.stream_applies(M, 151936, K, BF) for M in (1, 8, 16, 32)) and not ops.stream_applies(33, 151936, K, BF)
     assert not ops.stream_applies(8, 32768, 1024, BF) and ops.stream_applies(9, 32768, 1024, BF) and not ops.stream_applies(17, 32768, 1024, BF)
+    assert not ops.stream_applies(8, 16384, 200, BF) and ops.stream_applies(9, 16384, 200, BF) and ops.stream_applies(8, 65536, 200, BF)
     assert not ops.stream_applies(8, 151936, 1024, torch.float32) and not ops.stream_applies(8, 151936, 1020, BF)
     assert not any(ops.stream_applies(M, N, K, BF) for M in (1, 16, 32) for name in ("0.6b", "1.7b") for N, K in _products(name).values())
     glu = lambda M, name: ops.swiglu_stream_applies(M, SIZES[name][1], SIZES[name][0], BF)

@@ -190,22 +190,48 @@ def test_linear_tcgen05_swapped(M, N, K, out_f32, monkeypatch):
 @pytest.mark.parametrize("M", [1, 8, 16, 17, 32])
 @pytest.mark.parametrize("N,K", [(64, 64), (63, 8), (130, 200), (16391, 136), (28480, 1032)])
 @pytest.mark.parametrize("out_f32", [False, True])
-def test_linear_tcgen05_stream(M, N, K, out_f32, monkeypatch):
+@pytest.mark.parametrize("activation", [None, "relu_squared"])
+def test_linear_tcgen05_stream(M, N, K, out_f32, activation):
     """64 weight rows a CTA, up to 32 rows: edges in M, N (an odd number of rows, one CTA more than three per SM) and K (less
-    than half a stage, one half of the last one missing)."""
-    monkeypatch.setattr(ops, "STREAM_MIN_N", 1)
-    monkeypatch.setattr(ops, "STREAM_WIDE_MIN_N", 1)
-    assert ops.stream_applies(M, N, K, torch.bfloat16) or (N == 28480 and M <= 8)
+    than half a stage, one half of the last one missing), and an activation of the sums.  The form is asked for by itself:
+    ``linear`` takes it from some sizes on only."""
     x = _randn((M, K), torch.bfloat16, 18)
     w = _randn((N, K), torch.bfloat16, 19, 0.1)
-    odt = torch.float32 if out_f32 else torch.bfloat16
-    want = torch.empty(M, N, dtype=odt)
-    ref_ops.linear(x, w, want)
-    got = torch.full((M + 1, N), float("nan"), dtype=odt, device=DEV)
-    ops.linear(x.to(DEV), w.to(DEV), got[:M])
+    want = x.float() @ w.float().t()
+    if activation:
+        want = want.clamp(min=0) ** 2
+    got = torch.full((M + 1, N), float("nan"), dtype=torch.float32 if out_f32 else torch.bfloat16, device=DEV)
+    xd, wd = x.to(DEV), w.to(DEV)
+    ops._check(ops.lib().qe_linear_tcgen05_swap(ops._ptr(xd), ops._ptr(wd), ops._ptr(got), M, N, K,
+                                                int(out_f32) | ops.activation_code(activation) << 1, 1, 0, ops._stream()), "linear")
     torch.cuda.synchronize()
     assert ops.tcgen05_status() == 0 and got[M].isnan().all()
-    _close(got[:M], want, torch.bfloat16, scale=float(want.float().abs().max()))
+    # float32: a sum of K terms in another order, squared or not, is within (K + 8) 2^-23 of the terms' absolute sum (times twice
+    # the result where it is squared); bfloat16 adds half a unit of 2^-8
+    bound = (K + 8) * 2.0 ** -23 * (x.float().abs() @ w.float().abs().t())
+    if activation:
+        bound = bound * (2 * want.sqrt() + bound) + 2.0 ** -22 * want
+    if not out_f32:
+        bound = bound + 2.0 ** -8 * want.abs()
+    assert ((got[:M].float().cpu() - want).abs() <= bound + 1e-30).all()
+
+
+@pytest.mark.parametrize("M", [1, 8, 16])
+@pytest.mark.parametrize("N,K", [(16448, 1024), (16390, 4096), (16448, 520), (16384, 1096), (65536, 2560), (65530, 72), (50000, 1112)])
+def test_linear_of_few_rows_against_many_weight_rows_keeps_its_precision(M, N, K):
+    """Float32 results of up to 16 rows against 64 bits.  Tensor memory adds without rounding to nearest: a chain of c products of 16 k
+    loses half a unit (2^-24) of a sum on average, and the sums of a chain and the chains together are smaller than the result:
+    2^-25 a product; eight chains are added up to nearest.  (One chain over K was off by 1e-6 for K = 1 024, 4e-6 for 4 096.)"""
+    assert ops.stream_applies(M, N, K, torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(N + K + M)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    got = torch.empty(M, N, dtype=torch.float32, device=DEV)
+    ops.linear(x, w, got)
+    want = x.double() @ w.double().t()
+    chain = -(-(-(-K // 64)) // 8) * 4
+    err = float((got.double() - want).norm() / want.norm())
+    assert ops.tcgen05_status() == 0 and err <= chain * 2.0 ** -25 + 3 * 2.0 ** -24, err
 
 
 @pytest.mark.parametrize("M", [1, 15, 16, 31, 33, 64])
