@@ -257,7 +257,7 @@ def test_linear_swiglu_stream(M, I, K, activation):
     _close(got[:M], want, torch.bfloat16, scale=float(want.abs().max()), tol16=1e-2)
 
 
-@pytest.mark.parametrize("M", [1, 9, 17, 33, 64])
+@pytest.mark.parametrize("M", [1, 9, 16, 17, 32, 33, 64])
 @pytest.mark.parametrize("N,K,splits", [(1024, 2048, 8), (1024, 3072, 8), (1000, 1032, 4), (132, 200, 2), (4096, 1024, 4),
                                         (256, 192, 8), (6144, 1024, 2), (2560, 4096, 4)])
 @pytest.mark.parametrize("mode", ["bf16", "f32", "add"])
@@ -546,7 +546,7 @@ def test_linear_qkv_rope_small(T, Hq, Hkv, K, P, norm, angles, write_kv):
     assert float(flat[mask].abs().max()) == 0.0
 
 
-def _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed, spike=None):
+def _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed, spike=None, planes=2):
     """Build a paged cache with scattered pages for requests with ctx_lens[r] cached tokens and
     q_lens[r] new ones; returns everything both implementations need."""
     g = torch.Generator().manual_seed(seed)
@@ -561,7 +561,7 @@ def _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed, spike=
     for r in range(R):
         for b in range(blocks[r]):
             table[r, b] = next(it)
-    cache = (torch.randn(n_pages, 2, Hkv, P, D, generator=g)).to(dtype)
+    cache = (torch.randn(n_pages, planes, Hkv, P, D, generator=g)).to(dtype)
     T = sum(q_lens)
     qkv = torch.randn(T, (Hq + 2 * Hkv) * D, generator=g).to(dtype)
     if spike is not None:
@@ -581,24 +581,29 @@ def _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed, spike=
                 ctx=torch.tensor(ctx_lens, dtype=torch.int32), T=T)
 
 
-def _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, fn, dev, flash=True, uniform=None, arena=None):
+def _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, fn, dev, flash=True, uniform=None, arena=None, **options):
     """Run one implementation (``arena``: with that scratch memory, and the counters that belong to it).  On the GPU ``flash`` lets the step's plan carry the tensor-core
     kernel's work items (used when the kernel takes the geometry); without it the generic kernel runs.
-    ``uniform``: every request's context in that many parts, as in a decode step replayed from a graph."""
+    ``uniform``: every request's context in that many parts, as in a decode step replayed from a graph.  ``options``: what
+    ``paged_attention`` does to the scores and which values the weights meet."""
     from qwen_engine_b200.engine.runner import ModelRunner
     if arena is None:
         arena = Arena(dev)
     arena.reset()
     scale = 1.0 / math.sqrt(D)
-    geos = ((Hq, Hkv, D, window),) if (flash and dev != "cpu") else ()
+    planes = case["cache"].shape[1]
+    geo = (Hq, Hkv, D, window, "slopes" in options, planes) if planes > 2 or "slopes" in options else (Hq, Hkv, D, window)
+    geos = (geo[:5] if planes == 2 else geo,) if (flash and dev != "cpu") else ()
     plan = ops.plan_attention(list(q_lens), list(ctx_lens), P, geos, dtype,
                               uniform_splits={geos[0]: uniform} if uniform and geos else None)
     devplan = ModelRunner._device_plan(
         plan, {"plan_" + k: torch.tensor(v, dtype=torch.int32, device=dev) for k, v in plan.items()}, geos)
     ctx = SimpleNamespace(cu_q=case["cu_q"].to(dev), ctx_lens=case["ctx"].to(dev), attn_plan=devplan,
                           q_lens_host=list(q_lens), ctx_lens_host=list(ctx_lens), arena=arena)
-    out = torch.zeros(case["T"], Hq * D, dtype=dtype, device=dev)
-    fn(case["qkv"].to(dev), case["cache"].to(dev), case["table"].to(dev), ctx, out, scale, window, Hq, Hkv, D)
+    shifts = options.get("value_shifts", 1)
+    out = torch.zeros(*((shifts,) if shifts > 1 else ()), case["T"], Hq * (planes - 1) * D, dtype=dtype, device=dev)
+    options = {k: v.to(dev) if isinstance(v, torch.Tensor) else v for k, v in options.items()}
+    fn(case["qkv"].to(dev), case["cache"].to(dev), case["table"].to(dev), ctx, out, scale, window, Hq, Hkv, D, **options)
     if dev != "cpu":
         torch.cuda.synchronize()
     return out
@@ -628,6 +633,30 @@ def test_paged_attention(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, flash):
     want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ref_ops.paged_attention, "cpu")
     got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ops.paged_attention, DEV, flash=flash)
     _close(got, want, dtype, tol32=2e-5, tol16=1.6e-2)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("Hq,Hkv,D,P", [(4, 2, 6, 4), (3, 3, 30, 8), (4, 2, 129, 4), (2, 1, 257, 8), (4, 2, 8, 4), (4, 2, 64, 16), (2, 2, 260, 8)])
+@pytest.mark.parametrize("planes,options", [(2, {}), (2, dict(value_shift=1)), (3, {})])
+@pytest.mark.parametrize("off", [0, 1])
+def test_generic_attention_element_by_element(dtype, Hq, Hkv, D, P, planes, options, off):
+    """Heads whose size is no multiple of four, and queries and pages that start an element off a 16-byte boundary: the kernel
+    reads them element by element; values of the keys' own kv head, of another one, and in several blocks."""
+    if Hkv == 1:
+        options = {}
+    q_lens, ctx_lens = [37, 1, 5], [0, 70, 33]
+    case = _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, seed=64, planes=planes)
+    want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ref_ops.paged_attention, "cpu", **options)
+
+    def moved(t):                                       # the same values, `off` elements further on
+        buf = torch.empty(t.numel() + off, dtype=t.dtype, device=DEV)
+        buf[off:] = t.to(DEV).flatten()
+        return buf[off:].view(t.shape)
+    case = dict(case, qkv=moved(case["qkv"]), cache=moved(case["cache"]))
+    assert case["qkv"].data_ptr() % 16 == off * case["qkv"].element_size()
+    got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, 0, ops.paged_attention, DEV, flash=False, **options)
+    assert ops.last_attention_kernel == "paged_attention_generic"
+    _close(got, want, dtype)
 
 
 @pytest.mark.parametrize("Hq,Hkv,D,P", [(16, 8, 128, 16), (4, 1, 32, 8), (6, 2, 48, 4), (8, 1, 64, 16)])
@@ -751,6 +780,56 @@ def test_decode_attention_parts_by_length(Hq, Hkv, P, window, ctx_lens, total, d
         assert ops.last_attention_kernel == "decode_attention_mma"
         _close(got, want, dtype)
     assert int(arena.counters["fa"].abs().max()) == 0
+
+
+_SLOPES = 2.0 ** (-0.5 * torch.arange(1, 17))
+_SINKS = torch.linspace(-2.0, 3.0, 16)
+ATTENTION_OPTIONS = [
+    (0, 2, dict(slopes=_SLOPES)), (300, 2, dict(slopes=_SLOPES)), (0, 2, dict(softcap=1.5)), (0, 2, dict(sinks=_SINKS)),
+    (200, 2, dict(softcap=2.0, sinks=_SINKS)), (0, 2, dict(sinks=_SINKS, value_shift=3)),
+    (0, 2, dict(value_shifts=8)), (0, 2, dict(softcap=1.5, sinks=_SINKS, value_shifts=3)),
+    (0, 3, {}), (0, 4, dict(softcap=1.5, sinks=_SINKS)), (150, 3, dict(sinks=_SINKS)),
+]
+
+
+@pytest.mark.parametrize("window,planes,options", ATTENTION_OPTIONS)
+@pytest.mark.parametrize("ctx_lens,total", [([0, 15, 300, 2023, 47, 800, 31, 555, 1200, 16], 37), ([3] * 8 + [5000, 7], 74)])
+def test_decode_attention_parts_by_length_with_every_option(window, planes, options, ctx_lens, total, decode_kernel):
+    """What a decode step's lists by length (whole contexts, parts, items without rows) meet beside plain scores: a distance bias,
+    bent scores, sinks, other kv heads' values, all of them in one launch, several blocks of values."""
+    Hq, Hkv, D, P, dtype = 16, 8, 128, 16, torch.bfloat16
+    q_lens = [1] * len(ctx_lens)
+    case = _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed=62, planes=planes)
+    want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ref_ops.paged_attention, "cpu", **options)
+    arena = Arena(DEV)
+    for _ in range(2):                                  # (the second launch finds the counters as the first left them)
+        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV,
+                             uniform=ops.TotalParts(total), arena=arena, **options)
+        assert ops.last_attention_kernel == "decode_attention_mma"
+        _close(got, want, dtype)
+    assert int(arena.counters["fa"].abs().max()) == 0
+
+
+@pytest.mark.parametrize("window,planes,options", [(0, 2, {}), (1500, 2, {})] + ATTENTION_OPTIONS)
+def test_decoded_tokens_by_length_beside_a_prompt_portion(window, planes, options):
+    """A step whose prompt portion goes to the tcgen05 kernel and whose decoded tokens are cut by their lengths: the plan says so,
+    and every row is that of the plain reference."""
+    Hq, Hkv, D, P, dtype = 16, 8, 128, 16, torch.bfloat16
+    q_lens = [1] * 7 + [150] + [1] * 8
+    ctx_lens = [150 + 130 * i for i in range(7)] + [333] + [1100 + 130 * i for i in range(8)]
+    geo = (Hq, Hkv, D, window, "slopes" in options, planes)
+    info = ops.plan_attention(q_lens, ctx_lens, P, (geo,), dtype)
+    many = ops.FLASH_TARGET_CTAS // (Hkv * (planes - 1))
+    by_length = len(info["fa0_items"]) // ops.FLASH_ITEM_INTS in (many, 2 * many) and info["fa0_merge"] == []
+    assert "tc0_items" in info and by_length == (window in (0, 1500) and planes < 4)   # (short windows leave contexts of one length)
+    case = _attention_case(dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, seed=63, planes=planes)
+    want = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ref_ops.paged_attention, "cpu", **options)
+    arena = Arena(DEV)
+    for _ in range(2):
+        got = _run_attention(case, dtype, Hq, Hkv, D, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, arena=arena, **options)
+        assert ops.last_attention_kernel == "decode_attention_mma" and ops.tc_attention_status() == 0
+        _close(got, want, dtype)
+    assert all(not t.any() for t in arena.counters.values())
 
 
 def test_decode_attention_mma_asks_for_the_next_layers_cache(monkeypatch):
