@@ -16,7 +16,7 @@
 // Precision: tensor memory adds a product in without rounding to nearest, and the error grows with the length of the chain (1e-6 of
 // the result for K = 1 024 in one chain, 4e-6 for 4 096).  Up to 16 rows, where the weight-streaming product gives the k to eight
 // warps at most, every 64 k go to the next of eight accumulators of 16 columns, which are added up in order at the end: chains no
-// longer than there (151 936 x 1 024 1.3e-7, that product 2.2e-7; 16 384 x 4 096 both 4.8e-7).  It costs 0.5 us a round of CTAs.
+// longer than there (151 936 x 1 024 1.3e-7, that product 2.2e-7; 16 384 x 4 096 both 4.8e-7).  It costs 0.3-0.5 us a launch and 1.3 over the vocabulary.
 //
 // Six warps as in gemm_tcgen05_swap.cu: TMA, MMA, and four that read the accumulator (the 64-row form keeps row r in lane
 // r mod 16 of the quarter r / 16), put it into the ring's memory as [token][row] and store whole runs of a token's outputs.
@@ -150,29 +150,34 @@ gemm_tcgen05_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
     if (ok) {
 #pragma unroll 1
       for (int c0 = 0; c0 < mt; c0 += 16) {
-        constexpr int AT_ONCE = ACCS < 4 ? ACCS : 4;
-        float r[16];
-#pragma unroll
-        for (int a0 = 0; a0 < ACCS; a0 += AT_ONCE) {
-          if (a0 >= 2 * num_kb) break;                  // accumulators that no k reached hold nothing
-          uint32_t u[AT_ONCE][16];
-#pragma unroll
-          for (int a = 0; a < AT_ONCE; ++a) sr_load16(tmem + ((uint32_t)(quarter * 32) << 16) + (a0 + a) * BT + c0, u[a]);
+        uint32_t r[16];
+        if constexpr (ACCS == 1) {
+          sr_load16(tmem + ((uint32_t)(quarter * 32) << 16) + c0, r);
           tc_wait_ld();
+        } else {                                        // added in order, four at a time on their way
+          static_assert(ACCS == 8, "two rounds");
 #pragma unroll
-          for (int a = 0; a < AT_ONCE; ++a)
+          for (int a0 = 0; a0 < ACCS; a0 += 4) {
+            if (a0 >= 2 * num_kb) break;                // accumulators that no k reached hold nothing
+            uint32_t u[4][16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) asm volatile("" : "+r"(u[a][j]));      // (not read before the wait)
+            for (int a = 0; a < 4; ++a) sr_load16(tmem + ((uint32_t)(quarter * 32) << 16) + (a0 + a) * BT + c0, u[a]);
+            tc_wait_ld();
 #pragma unroll
-          for (int a = 0; a < AT_ONCE; ++a) {
-            const bool any = a0 + a < 2 * num_kb;
+            for (int a = 0; a < 4; ++a) {
+              const bool any = a0 + a < 2 * num_kb;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) r[j] = a0 + a == 0 ? __uint_as_float(u[a][j]) : r[j] + (any ? __uint_as_float(u[a][j]) : 0.f);
+              for (int j = 0; j < 16; ++j) {
+                asm volatile("" : "+r"(u[a][j]));       // (not read before the wait)
+                if (a0 + a == 0) r[j] = u[a][j];
+                else r[j] = __float_as_uint(__uint_as_float(r[j]) + (any ? __uint_as_float(u[a][j]) : 0.f));
+              }
+            }
           }
         }
         if (lane < 16) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) sums[(c0 + j) * SR_BM + quarter * 16 + lane] = r[j];
+          for (int j = 0; j < 16; ++j) sums[(c0 + j) * SR_BM + quarter * 16 + lane] = __uint_as_float(r[j]);
         }
       }
     }
