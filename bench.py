@@ -331,6 +331,9 @@ def kernel_chains(loaded, cfg, peaks, tag, ctx, torch, ops, out) -> None:
     if not dec and ops.swiglu_fused_applies(T, I, H, bf):
         us = chain(lambda: [ops.linear_swiglu(x, f.w_gate_up, act) for f in ffns])
         record(f"{tag}_gate_up_swiglu", us, flops=2.0 * T * 2 * I * H)
+    elif dec and ops.swiglu_stream_applies(T, I, H, bf):
+        us = chain(lambda: [ops.linear_swiglu_stream(x, f.w_gate_up, act) for f in ffns])
+        record(f"{tag}_gate_up_swiglu", us, nbytes=2 * I * H * 2)
     elif dec and ops.swiglu_small_applies(T, I, H, bf):
         us = chain(lambda: [ops.linear_swiglu_small(x, f.w_gate_up, act) for f in ffns])
         record(f"{tag}_gate_up_swiglu", us, nbytes=2 * I * H * 2)
@@ -459,7 +462,7 @@ COMPARE_SIZES = {
     "w2048": dict(width=2048, ff=6144, heads=16, kv_heads=8, head_dim=128, gla_heads=16, gla_dk=64, gla_dv=128, window=1024,
                   layers=8, vocab=32768, preset="qwen3-1.7b"),
 }
-_TIMED_OPS = ("embedding", "linear", "linear_swiglu", "linear_swiglu_small", "linear_silu_mul", "linear_qkv_rope", "act_mul",
+_TIMED_OPS = ("embedding", "linear", "linear_swiglu", "linear_swiglu_small", "linear_swiglu_stream", "linear_silu_mul", "linear_qkv_rope", "act_mul",
               "qk_norm_rope_kv_write", "paged_attention", "channel_decay", "linear_attention_scan", "head_norm_gate",
               "add_rmsnorm", "add_rmsnorm_rows", "rope_table", "latent_prepare", "head_linear", "short_conv", "unit_norm",
               "delta_rule_scan", "moe_route", "moe_experts", "qk_bias_norm_kv_write", "stream_conv", "gated_norm_add",

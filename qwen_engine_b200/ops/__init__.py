@@ -28,7 +28,8 @@ SMALL_M_MAX = 64        # rows up to which the weight-streaming product is used
 SPLITK = True           # products of some tens of rows by clusters of CTAs that share K (gemm_tcgen05_splitk.cu)
 SPLITK_MIN_M = 17       # rows from which, up to SPLITK_MAX_M, that kernel serves
 SPLITK_MAX_M = 64
-SPLITK_MAX_CTAS = 148   # clusters x CTAs at most: all on the GPU at once
+SPLITK_MAX_CTAS = 148   # tiles of 128 weight rows x CTAs per cluster at most: all on the GPU at once (up to 32 rows clusters of
+                        # 2 and 4 take tiles of 64, twice as many CTAs of half the shared memory, two per SM)
 SPLITK_LONG_K = 4096    # K from which that kernel serves from SPLITK_LONG_K_MIN_M rows on, where the weight rows / 16 exceed the SMs (0: never)
 SPLITK_LONG_K_MIN_M = 9
 SPLITK_VERY_LONG_K = 8192   # K from which, under the same conditions, every number of rows goes there (Qwen3-4B's down product)
@@ -400,9 +401,10 @@ def _linear_normed(x: NormedInput, w: torch.Tensor, out: torch.Tensor) -> bool:
 
 
 def splitk_splits(M: int, N: int, K: int, dtype: torch.dtype) -> int:
-    """How many CTAs share a tile of 128 weight rows, each with a share of K, in the product of some tens
-    of rows (``linear_splitk``): as many of 8, 4, 2 as keep all clusters on the GPU at once (8 only for few clusters); 0 where that
-    kernel does not apply (few rows, enough weight rows for every SM, other types)."""
+    """How many CTAs share a tile of weight rows, each with a share of K, in the product of some tens
+    of rows (``linear_splitk``): as many of 8, 4, 2 as keep all clusters on the GPU at once (8 only for few clusters), counted in tiles
+    of 128 rows and with two blocks of 64 k for each; 0 where that kernel does not apply (few rows, enough weight rows for every
+    SM, other types)."""
     if not (TCGEN05_ENABLED and SPLITK and dtype == torch.bfloat16 and M <= SPLITK_MAX_M and K % 8 == 0 and N % 4 == 0):
         return 0
     # From 9 rows on already (from the first, where K is very long) where the streaming kernel is at its worst: more CTAs of 16 weight rows than SMs (they do not
@@ -422,7 +424,7 @@ def splitk_splits(M: int, N: int, K: int, dtype: torch.dtype) -> int:
 
 def linear_splitk(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: int, add: bool = False,
                   activation: Optional[str] = None) -> None:
-    """``linear`` in bfloat16 for up to 64 rows by clusters of ``splits`` CTAs that share 128 weight rows
+    """``linear`` in bfloat16 for up to 64 rows by clusters of ``splits`` CTAs that share 64 or 128 weight rows
     and meet through distributed shared memory; ``add``: out (float32) += the product."""
     _need(not (add and activation), "linear_splitk: a product that is added to the stream has no activation")
     M, K = x.shape
