@@ -13,11 +13,12 @@
 //  - a thread keeps TM x TN pairs of sums and reads 4 k of a row in one load: the pair (k, k + 1) is the register pair that
 //    the two-wide fma takes, so nothing is packed or duplicated; up to 8 x 4 sums, since a 16-byte load from shared memory
 //    costs four of its cycles even where lanes read the same word;
-//  - up to 16 rows the four groups are warps of their own, so that a tile has enough of them to hide its loads (a block is 64
+//  - in tiles of up to 16 rows the four groups are warps of their own, so that a tile has enough of them to hide its loads (a block is 64
 //    k, a run of each); beyond, a thread takes one group after the other (a block is two runs of a group);
 //  - tiles are 64 weight rows, and a cluster of S CTAs shares K where the tiles alone would leave SMs idle; the partial
 //    tiles meet through distributed shared memory, each CTA finishing a share of the outputs;
-//  - the tile's height is the smallest of 4, 8, 16 that takes all rows, beyond that the one of 32, 48, 64 that wastes least.
+//  - the tile's height is the smallest of 4, 8, 16 that takes all rows, beyond that the one of 32, 48, 64 that wastes least (K up
+//    to 64: 16 or 48).
 // Measured on a B200, chains of launches over weights larger than L2: 4096 x 1024 at 3 rows 5.5 us (3.1 TB/s), 151936 x 1024
 // at 3 rows 99 us (6.3 TB/s), 6144 x 1024 at 141 rows 57 us (31 TFLOP/s).  With two threads' worth of k in one group and
 // four rows of one column a thread, 3 rows took 7.3 and 186 us; 8 x 8 sums a thread from 32 rows on (8 warps an SM instead
