@@ -1201,3 +1201,21 @@ def test_linear_small_m_shares_k_in_clusters(M, N, K, mode, rows8, monkeypatch):
         out = torch.empty(M, N, dtype=torch.float32 if mode == "f32" else torch.bfloat16, device=DEV)
         ops.linear(x.to(DEV), w.to(DEV), out)
         _close(out, want, torch.bfloat16)
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,P", [(16, 8, 128, 16), (4, 2, 64, 8), (6, 2, 256, 16), (6, 2, 48, 4)])
+@pytest.mark.parametrize("n,ctx", [(9, 300), (20, 700), (31, 2100), (23, 9000)])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_portions_of_some_rows_behind_long_contexts(Hq, Hkv, D, P, n, ctx, sinks):
+    """A portion of more rows than the decode kernel takes and fewer than the tcgen05 kernel does: its context is cut into parts (2 to more than 8, an
+    odd number of places for the merging threads) that the last CTA adds up."""
+    if n * (Hq // Hkv) > 64:
+        n = 64 // (Hq // Hkv) - 1
+    options = dict(sinks=torch.linspace(-1.0, 2.0, Hq)) if sinks else {}
+    plan = ops.plan_attention([n], [ctx], P, ((Hq, Hkv, D, 0),), torch.bfloat16)
+    assert plan["fa0_info"][0] >= 2 and plan["fa0_info"][3] > 16 and (ctx < 5000 or plan["fa0_info"][0] > 8)
+    case = _attention_case(torch.bfloat16, Hq, Hkv, D, P, [n], [ctx], 0, seed=86)
+    want = _run_attention(case, torch.bfloat16, Hq, Hkv, D, P, [n], [ctx], 0, ref_ops.paged_attention, "cpu", **options)
+    got = _run_attention(case, torch.bfloat16, Hq, Hkv, D, P, [n], [ctx], 0, ops.paged_attention, DEV, **options)
+    assert ops.last_attention_kernel == "flash_attention"
+    _close(got, want, torch.bfloat16)
