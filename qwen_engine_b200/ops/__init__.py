@@ -1272,8 +1272,16 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
             else:
                 lo = (max(0, c - window + 1) // FLASH_BN) * FLASH_BN if window else 0
                 splits = 1
+        most_parts = max(1, FLASH_TARGET_CTAS // max(1, base))
+        if (uniform_splits is None and rest and len(rest) == len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_WIDE and D == 128
+                and geometry_planes(geo) >= 2 and base <= TC_TARGET_CTAS and max(q_lens) * G <= 16):
+            # a few tokens of every request, nothing else: CTAs of 8 warps, one per SM, and parts that form clusters, as for decoded
+            # tokens (7 requests of one token and one of three behind 1 300 keys, 12 rows: 24.9 us in 4 parts of 4 warps, of
+            # which two with their in-boxes do not fit an SM, 12.9 in 2 parts of 8)
+            span = max(attended_keys(q_lens, ctx_lens, window))
+            most_parts = _cluster_parts(max(1, min(TC_TARGET_CTAS // base, -(-span // FLASH_SPLIT))), base, span)
                 if n <= tpt and base < FLASH_TARGET_CTAS and total - lo > FLASH_SPLIT:
-                    splits = min(-(-(total - lo) // FLASH_SPLIT), max(1, FLASH_TARGET_CTAS // base))
+                    splits = min(-(-(total - lo) // FLASH_SPLIT), most_parts)
             if splits > 1:
                 for sp in range(splits):
                     item = [r, 0, 0, 0, n_parts + sp, splits, sp, row0, n, c, 0, 0]
@@ -1340,24 +1348,30 @@ def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype
             out[geo] = parts
             continue
         if (DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_WIDE and dtype == torch.bfloat16 and D == 128
+def _cluster_parts(parts: int, ctas: int, span: int) -> int:
+    """The number of parts near ``parts`` that ``ctas`` CTAs of 8 warps are best cut into for contexts of up to ``span`` keys.
+    2, 4 or 8 parts of a request form a thread-block cluster and meet on chip, which beats the merge through
+    global memory (measured at 0.6B sizes, context 1 024: 2 requests in 4 parts each 0.80 ms a step, in 5
+    parts 0.95); clusters of 8 only while all of them still fit the GPU at once (at most 8 of them: 0.95 ms
+    with 16 of them) or where 4 parts would be long ones."""
+    if not DECODE_ATTENTION_CLUSTERS or parts <= 2:
+        return parts
+    few = ctas * 8 <= 64
+    if parts == 3:
+        return 4 if ctas * 4 <= TC_TARGET_CTAS else 2
+    if parts < 8:
+        return 8 if few else 4
+    if few or (parts == 8 and span > DECODE_CLUSTER4_MAX_SPAN):
+        return 8
+    return 4 if span <= DECODE_CLUSTER4_MAX_SPAN else parts
+
+
                 and Hq // Hkv <= 16 and num_reqs * Hkv <= TC_TARGET_CTAS):
             target = TC_TARGET_CTAS                                       # one CTA of 8 warps per SM
         want = max(1, target // max(1, num_reqs * Hkv))                   # all parts run in one wave
         parts = max(1, min(want, -(-span // FLASH_SPLIT)))
-        if target == TC_TARGET_CTAS and DECODE_ATTENTION_CLUSTERS and parts > 2:
-            # 2, 4 or 8 parts of a request form a thread-block cluster and meet on chip, which beats the merge through
-            # global memory (measured at 0.6B sizes, context 1 024: 2 requests in 4 parts each 0.80 ms a step, in 5
-            # parts 0.95); clusters of 8 only while all of them still fit the GPU at once (at most 8 of them: 0.95 ms
-            # with 16 of them) or where 4 parts would be long ones
-            few = num_reqs * Hkv * 8 <= 64
-            if parts == 3:
-                parts = 4 if num_reqs * Hkv * 4 <= target else 2
-            elif parts < 8:
-                parts = 8 if few else 4
-            elif few or (parts == 8 and span > DECODE_CLUSTER4_MAX_SPAN):
-                parts = 8
-            elif span <= DECODE_CLUSTER4_MAX_SPAN:
-                parts = 4
+        if target == TC_TARGET_CTAS:
+            parts = _cluster_parts(parts, num_reqs * Hkv, span)
         out[geo] = parts
         if (ctx_lens and parts == 1 and DECODE_ATTENTION_MMA and dtype == torch.bfloat16 and D == 128 and Hq // Hkv <= 16
                 and geometry_planes(geo) >= 2):

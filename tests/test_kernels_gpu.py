@@ -1219,3 +1219,20 @@ def test_portions_of_some_rows_behind_long_contexts(Hq, Hkv, D, P, n, ctx, sinks
     got = _run_attention(case, torch.bfloat16, Hq, Hkv, D, P, [n], [ctx], 0, ops.paged_attention, DEV, **options)
     assert ops.last_attention_kernel == "flash_attention"
     _close(got, want, torch.bfloat16)
+
+
+@pytest.mark.parametrize("Hq,Hkv,q_lens,ctx_lens,parts", [
+    (32, 8, [1] * 7 + [3], [1300 + 16 * i for i in range(7)] + [1024], 2),
+    (16, 8, [2, 5], [900, 1000], 4), (16, 8, [8], [2100], 8), (32, 8, [4] * 18, [700] * 18, 1), (16, 8, [1, 2, 1], [40, 3000, 700], 0),
+])
+def test_a_few_tokens_of_every_request_in_clusters(Hq, Hkv, q_lens, ctx_lens, parts):
+    """Steps of 1 to 8 tokens a request: as many parts as CTAs of 8 warps fit the SMs once, in clusters where all requests have as many
+    (0: they do not)."""
+    P, dtype = 16, torch.bfloat16
+    info = ops.plan_attention(q_lens, ctx_lens, P, ((Hq, Hkv, 128, 0),), dtype)["fa0_info"]
+    assert info[4] == (parts if parts > 1 else 0) and info[0] == (parts * len(q_lens) if parts > 1 else info[0])
+    case = _attention_case(dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, 0, seed=87)
+    want = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, 0, ref_ops.paged_attention, "cpu")
+    got = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, 0, ops.paged_attention, DEV)
+    assert ops.last_attention_kernel == "decode_attention_mma"
+    _close(got, want, dtype)
