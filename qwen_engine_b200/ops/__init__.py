@@ -1250,6 +1250,14 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
                 keys = attended_keys([q_lens[r] for r in rest], [ctx_lens[r] for r in rest], window)
                 items_in_all = parts_for_lengths(geo, keys, max(-(-k // min(-(-k // FLASH_SPLIT), at_most)) for k in keys),
                                                  max(q_lens[r] for r in rest) * G)
+        most_parts = max(1, FLASH_TARGET_CTAS // max(1, base))
+        if (uniform_splits is None and rest and len(rest) == len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_WIDE and D == 128
+                and geometry_planes(geo) >= 2 and base <= TC_TARGET_CTAS and max(q_lens) * G <= 16):
+            # a few tokens of every request, nothing else: CTAs of 8 warps, one per SM, and parts that form clusters, as for decoded
+            # tokens (7 requests of one token and one of three behind 1 300 keys, 12 rows: 24.9 us in 4 parts of 4 warps, of
+            # which two with their in-boxes do not fit an SM, 12.9 in 2 parts of 8)
+            span = max(attended_keys(q_lens, ctx_lens, window))
+            most_parts = _cluster_parts(max(1, min(TC_TARGET_CTAS // base, -(-span // FLASH_SPLIT))), base, span)
         if items_in_all is not None:
             dealt = items_in_all.shares
             if dealt is None:
@@ -1272,14 +1280,6 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
             else:
                 lo = (max(0, c - window + 1) // FLASH_BN) * FLASH_BN if window else 0
                 splits = 1
-        most_parts = max(1, FLASH_TARGET_CTAS // max(1, base))
-        if (uniform_splits is None and rest and len(rest) == len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_WIDE and D == 128
-                and geometry_planes(geo) >= 2 and base <= TC_TARGET_CTAS and max(q_lens) * G <= 16):
-            # a few tokens of every request, nothing else: CTAs of 8 warps, one per SM, and parts that form clusters, as for decoded
-            # tokens (7 requests of one token and one of three behind 1 300 keys, 12 rows: 24.9 us in 4 parts of 4 warps, of
-            # which two with their in-boxes do not fit an SM, 12.9 in 2 parts of 8)
-            span = max(attended_keys(q_lens, ctx_lens, window))
-            most_parts = _cluster_parts(max(1, min(TC_TARGET_CTAS // base, -(-span // FLASH_SPLIT))), base, span)
                 if n <= tpt and base < FLASH_TARGET_CTAS and total - lo > FLASH_SPLIT:
                     splits = min(-(-(total - lo) // FLASH_SPLIT), most_parts)
             if splits > 1:
@@ -1326,6 +1326,24 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
 DECODE_CLUSTER4_MAX_SPAN = 4096   # keys up to which 4 parts in a cluster are preferred to more parts merged through memory
 
 
+def _cluster_parts(parts: int, ctas: int, span: int) -> int:
+    """The number of parts near ``parts`` that ``ctas`` CTAs of 8 warps are best cut into for contexts of up to ``span`` keys.
+    2, 4 or 8 parts of a request form a thread-block cluster and meet on chip, which beats the merge through
+    global memory (measured at 0.6B sizes, context 1 024: 2 requests in 4 parts each 0.80 ms a step, in 5
+    parts 0.95); clusters of 8 only while all of them still fit the GPU at once (at most 8 of them: 0.95 ms
+    with 16 of them) or where 4 parts would be long ones."""
+    if not DECODE_ATTENTION_CLUSTERS or parts <= 2:
+        return parts
+    few = ctas * 8 <= 64
+    if parts == 3:
+        return 4 if ctas * 4 <= TC_TARGET_CTAS else 2
+    if parts < 8:
+        return 8 if few else 4
+    if few or (parts == 8 and span > DECODE_CLUSTER4_MAX_SPAN):
+        return 8
+    return 4 if span <= DECODE_CLUSTER4_MAX_SPAN else parts
+
+
 def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype, ctx_lens: Optional[list] = None) -> dict:
     """The fixed number of parts per request for a decode step of ``num_reqs`` requests whose block
     tables hold up to ``max_tokens`` tokens: enough parts to fill the GPU, none shorter than a split.
@@ -1348,24 +1366,6 @@ def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype
             out[geo] = parts
             continue
         if (DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_WIDE and dtype == torch.bfloat16 and D == 128
-def _cluster_parts(parts: int, ctas: int, span: int) -> int:
-    """The number of parts near ``parts`` that ``ctas`` CTAs of 8 warps are best cut into for contexts of up to ``span`` keys.
-    2, 4 or 8 parts of a request form a thread-block cluster and meet on chip, which beats the merge through
-    global memory (measured at 0.6B sizes, context 1 024: 2 requests in 4 parts each 0.80 ms a step, in 5
-    parts 0.95); clusters of 8 only while all of them still fit the GPU at once (at most 8 of them: 0.95 ms
-    with 16 of them) or where 4 parts would be long ones."""
-    if not DECODE_ATTENTION_CLUSTERS or parts <= 2:
-        return parts
-    few = ctas * 8 <= 64
-    if parts == 3:
-        return 4 if ctas * 4 <= TC_TARGET_CTAS else 2
-    if parts < 8:
-        return 8 if few else 4
-    if few or (parts == 8 and span > DECODE_CLUSTER4_MAX_SPAN):
-        return 8
-    return 4 if span <= DECODE_CLUSTER4_MAX_SPAN else parts
-
-
                 and Hq // Hkv <= 16 and num_reqs * Hkv <= TC_TARGET_CTAS):
             target = TC_TARGET_CTAS                                       # one CTA of 8 warps per SM
         want = max(1, target // max(1, num_reqs * Hkv))                   # all parts run in one wave
