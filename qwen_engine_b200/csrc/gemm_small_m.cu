@@ -13,8 +13,9 @@
 // fixed order.  Any N; K a multiple of 8 (16-byte rows); the launcher refuses the rest.
 #include "gemm_small_m.cuh"
 
-template <int MT, typename TOut, int XMODE, bool RESID, int ROWS = 16>
-__global__ void __launch_bounds__(512)
+// PER_SM: CTAs of 8 warps that an SM has registers for (0: up to 16 warps, one CTA or more).
+template <int MT, typename TOut, int XMODE, bool RESID, int ROWS = 16, int PER_SM = 0>
+__global__ void __launch_bounds__(PER_SM ? 256 : 512, PER_SM)
 gemm_small_m_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                     TOut* __restrict__ out, int M, int N, int K, int k_per_warp, FuseArgs na) {
   extern __shared__ float red[];                    // [warps][16][8 MT]
@@ -206,6 +207,21 @@ static int launch_small_m(const void* x, const void* w, void* out, int M, int N,
     if (!RESID)
       cudaFuncSetAttribute(gemm_small_m_kernel<MT, __nv_bfloat16, XMODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
     configured = true;
+  }
+  if constexpr (MT == 1 && XMODE == X_PLAIN && !RESID) {
+    // More CTAs than two per SM: with 82 registers a thread only two of 8 warps fit, and what was left over waited for
+    // a second round (6 144 x 2 560, 384 CTAs, at 1 and 8 rows 10.4 and 11.4 us, with 80 registers 7.8 and 8.1; 5 120 x 1 024
+    // 4.9 and 5.2, now 2.8 and 3.0).
+    if (ctas > 2 * 148 && warps <= 8) {
+      if (out_f32)
+        qe_launch(gemm_small_m_kernel<MT, float, XMODE, RESID, 16, 3>, dim3(ctas), dim3(warps * 32), smem, stream,
+                  (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (float*)out, M, N, K, k_per_warp, na);
+      else
+        qe_launch(gemm_small_m_kernel<MT, __nv_bfloat16, XMODE, RESID, 16, 3>, dim3(ctas), dim3(warps * 32), smem, stream,
+                  (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, M, N, K, k_per_warp, na);
+      QE_CHECK_LAUNCH("linear_small_m");
+      return 0;
+    }
   }
   if (out_f32 || RESID) {
     qe_launch(gemm_small_m_kernel<MT, float, XMODE, RESID>, dim3(ctas), dim3(warps * 32), smem, stream,

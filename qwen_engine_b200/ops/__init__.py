@@ -506,6 +506,28 @@ def stream_applies(M: int, N: int, K: int, dtype: torch.dtype) -> bool:
     return N >= STREAM_MIN_N and (M > 8 or not (1 < rounds < 1.5 or (K < 512 and rounds < 1)))
 
 
+def few_rows_splits(M: int, N: int, K: int, dtype: torch.dtype) -> int:
+    """How many CTAs share K in a product of up to 16 rows that the weight-streaming product serves badly, beyond those that
+    ``splitk_splits`` names; 0: none.  That product's CTAs take 16 weight rows; three of them fit an SM, more wait for a
+    second round, and from 9 rows on an instruction covers two tiles of tokens.  Measured on a B200 (a chain of launches over
+    weights beyond L2; streaming / clusters), 9 and 16 rows: in clusters of 4 2 432 x 1 536 4.6, 5.0 / 4.3, 4 096 x 2 048 6.3,
+    6.8 / 5.6, 4 096 x 4 096 10.8, 12.0 / 8.3, but x 1 024 3.8, 4.1 / 4.3, and 4 736 x 2 048 6.4 / 9.2 (74 clusters of 4 do not all
+    find room); in clusters of 2 6 144 x 2 560 9.3, 9.8 / 7.9, but 5 120 x 2 048 6.5, 7.2 / 7.1; more than three CTAs per SM,
+    7 168 x 1 024 7.3, 7.8 / 5.1, 8 192 x 2 560 16.2, 17.7 / 9.0.  At 1 and 8 rows 8 192 x 1 536 8.4, 8.9 / 6.4, 6 144 x 4 096 11.8,
+    13.3 / 10.9, but 9 216 x 1 024 5.4 / 6.0 and 5 120 x 4 096 9.3, 9.9 / 10.1."""
+    if not (TCGEN05_ENABLED and SPLITK and dtype == torch.bfloat16 and 1 <= M <= 16 and K % 8 == 0 and N % 4 == 0):
+        return 0
+    ctas, tiles = -(-N // 16), -(-N // 128)
+    rounds = ctas > 3 * SPLITK_MAX_CTAS
+    if M > 8 and ctas > SPLITK_MAX_CTAS and tiles <= 32:
+        return 4 if K >= 1536 else 0
+    if M > 8:
+        gains = tiles > 32 and K >= (1024 if rounds else 2560)
+    else:
+        gains = K >= (1536 if rounds else 4096) and ctas >= 384
+    return 2 if gains and 2 * tiles <= SPLITK_MAX_CTAS else 0
+
+
 def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = None) -> None:
     """out[M, N] = x[M, K] · w[N, K]^T, float32 accumulation; out in x's dtype or float32.
     ``x`` may be a NormedInput (see there).  ``activation`` (``ACTIVATIONS``) is applied to the float32 sums in the
@@ -530,7 +552,7 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = No
         # very many weight rows (a vocabulary): all SMs stream them, 64 a CTA
         _check(lib().qe_linear_tcgen05_swap(_ptr(x), _ptr(w), _ptr(out), M, N, K, out_mode, 1, 0, _stream()), "linear")
         return
-    splits = splitk_splits(M, N, K, x.dtype)
+    splits = splitk_splits(M, N, K, x.dtype) or few_rows_splits(M, N, K, x.dtype)
     if splits:
         linear_splitk(x, w, out, splits, activation=activation)
         return

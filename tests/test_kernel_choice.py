@@ -76,3 +76,17 @@ def test_rows_beyond_what_a_form_serves_are_refused():
     for M, form, most in ((33, 1, b"32"), (64, 1, b"32"), (65, 2, b"64"), (257, 0, b"256")):
         assert call(M, form) == 1 and b"above " + most in ops.lib().qe_last_error()
     assert call(8, 3) == 1 and ops.STREAM_MAX_M == 32 and ops.STREAM_GLU_MAX_M == 64
+
+
+def test_few_rows_share_k_where_the_streaming_kernel_takes_a_second_round_or_two_tiles_of_tokens():
+    got = lambda M, N, K: ops.few_rows_splits(M, N, K, BF)
+    assert got(9, 2432, 1536) == got(16, 4096, 4096) == 4 and got(9, 4096, 1024) == 0 and got(9, 2368, 2048) == 0
+    assert got(9, 4736, 2048) == 0 and got(16, 6144, 2560) == 2 and got(16, 6144, 2048) == 0 and got(9, 7168, 1024) == 2
+    assert got(8, 8192, 1536) == got(1, 6144, 4096) == 2 and got(8, 9216, 1024) == got(8, 5120, 4096) == got(8, 6144, 2560) == 0
+    assert got(17, 6144, 2560) == got(8, 9600, 2560) == got(9, 12288, 2048) == 0          # (more than 74 clusters of 2)
+    assert ops.few_rows_splits(9, 6144, 2560, torch.float32) == 0 and got(9, 6144, 2564) == 0 and got(9, 6146, 2560) == 0
+    for M in (1, 8, 9, 16):
+        for N in range(16, 20000, 52):
+            for K in (512, 1024, 1536, 2048, 4096, 9728):
+                s = got(M, N, K)
+                assert s == 0 or (-(-N // 128) * s <= ops.SPLITK_MAX_CTAS and -(-K // 64) >= 2 * s)

@@ -1203,6 +1203,21 @@ def test_linear_small_m_shares_k_in_clusters(M, N, K, mode, rows8, monkeypatch):
         _close(out, want, torch.bfloat16)
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(4737, 72), (4800, 200), (7104, 1032), (7112, 1024), (2436, 1536), (4096, 1544), (6144, 2560), (6148, 4096)])
+@pytest.mark.parametrize("out_f32", [False, True])
+def test_linear_of_few_rows_against_more_than_a_round_of_weights(M, N, K, out_f32):
+    """Three CTAs of 16 weight rows per SM, and beyond that, or where K is long, clusters that share it."""
+    x, w = _randn((M, K), torch.bfloat16, 84), _randn((N, K), torch.bfloat16, 85, K ** -0.5)
+    odt = torch.float32 if out_f32 else torch.bfloat16
+    want = (x.double() @ w.double().t()).to(odt)
+    got = torch.full((M, N), float("nan"), dtype=odt, device=DEV)
+    ops.linear(x.to(DEV), w.to(DEV), got)
+    torch.cuda.synchronize()
+    assert ops.tcgen05_status() == 0
+    _close(got, want, odt, tol16=8e-3)
+
+
 @pytest.mark.parametrize("Hq,Hkv,D,P", [(16, 8, 128, 16), (4, 2, 64, 8), (6, 2, 256, 16), (6, 2, 48, 4)])
 @pytest.mark.parametrize("n,ctx", [(9, 300), (20, 700), (31, 2100), (23, 9000)])
 @pytest.mark.parametrize("sinks", [False, True])
