@@ -552,7 +552,8 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, activation: Optional[str] = No
         # very many weight rows (a vocabulary): all SMs stream them, 64 a CTA
         _check(lib().qe_linear_tcgen05_swap(_ptr(x), _ptr(w), _ptr(out), M, N, K, out_mode, 1, 0, _stream()), "linear")
         return
-    splits = splitk_splits(M, N, K, x.dtype) or few_rows_splits(M, N, K, x.dtype)
+    # (the clusters store pieces of 16 bytes; the weight-streaming product takes an output at any place)
+    splits = splitk_splits(M, N, K, x.dtype) or (few_rows_splits(M, N, K, x.dtype) if out.data_ptr() % 16 == 0 else 0)
     if splits:
         linear_splitk(x, w, out, splits, activation=activation)
         return

@@ -1211,11 +1211,12 @@ def test_linear_of_few_rows_against_more_than_a_round_of_weights(M, N, K, out_f3
     x, w = _randn((M, K), torch.bfloat16, 84), _randn((N, K), torch.bfloat16, 85, K ** -0.5)
     odt = torch.float32 if out_f32 else torch.bfloat16
     want = (x.double() @ w.double().t()).to(odt)
-    got = torch.full((M, N), float("nan"), dtype=odt, device=DEV)
-    ops.linear(x.to(DEV), w.to(DEV), got)
-    torch.cuda.synchronize()
-    assert ops.tcgen05_status() == 0
-    _close(got, want, odt, tol16=8e-3)
+    for off in (0, 2):                                  # (elements: an output off a 16-byte boundary is served too)
+        got = torch.full((M * N + off,), float("nan"), dtype=odt, device=DEV)[off:].view(M, N)
+        ops.linear(x.to(DEV), w.to(DEV), got)
+        torch.cuda.synchronize()
+        assert ops.tcgen05_status() == 0
+        _close(got, want, odt, tol16=8e-3)
 
 
 @pytest.mark.parametrize("Hq,Hkv,D,P", [(16, 8, 128, 16), (4, 2, 64, 8), (6, 2, 256, 16), (6, 2, 48, 4)])
