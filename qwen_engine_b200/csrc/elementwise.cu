@@ -156,75 +156,92 @@ __global__ void add_rmsnorm_bf16x8_kernel(float* __restrict__ resid, const __nv_
   }
 }
 
-// The same with one warp per row, for widths that are multiples of 256 up to 2048: a lane keeps its
-// NC pieces of 8 elements in registers between the sum of squares and the scaling, all its loads are
-// in flight together, and no block-wide barrier is needed.
-template <int NC>
-__global__ void add_rmsnorm_bf16_warp_kernel(float* __restrict__ resid, const __nv_bfloat16* __restrict__ delta,
-                                             const int* __restrict__ rows, const float* __restrict__ w,
-                                             float eps, __nv_bfloat16* __restrict__ out, int n_rows) {
-  constexpr int H = NC * 256;
+// The same with the row in registers, for widths NV x 128 x WARPS: a CTA of WARPS warps per row, a thread keeps its NV
+// pieces of 4 elements between the sum of squares and the scaling and has all its loads on their way together.  What
+// bounds it is the traffic through L2 (the row's four arrays are on the chip) and, with few rows, one round trip: a
+// warp's access is one run of 512 bytes (of 256 in bfloat16).  (A warp per row with 8 elements a lane touched every 32-byte
+// sector of the stream twice.)  Measured on a B200, a chain of launches, that form / this one: 1 024 wide 1.87 / 1.29 us at 8 rows, 5.71 /
+// 3.43 at 2 048 (25 MB through L2); 2 048 wide 5.64 / 3.19 at 527; 2 560 wide, two passes over the row
+// in add_rmsnorm_bf16x8_kernel, 2.64 / 1.56 at 16 and 10.65 / 6.39 at 2 048.
+__device__ __forceinline__ float4 ld_four(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ld_four(const __nv_bfloat16* p) {
+  const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p));
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+__device__ __forceinline__ void st_four(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void st_four(__nv_bfloat16* p, const float4& v) {
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+
+template <typename T, int NV, int WARPS, int ROWS>
+__global__ void __launch_bounds__(WARPS * 32 * ROWS)
+add_rmsnorm_row_kernel(float* __restrict__ resid, const T* __restrict__ delta, const int* __restrict__ rows,
+                       const float* __restrict__ w, float eps, T* __restrict__ out, int n_rows) {
+  static_assert(ROWS == 1 || WARPS == 1, "several rows a CTA: a warp each, which meets no barrier");
+  constexpr int H = NV * 128 * WARPS, STEP = WARPS * 128;             // STEP: elements between a thread's pieces
+  __shared__ float s_part[WARPS];
   pdl_launch_dependents();
-  const int lane = threadIdx.x & 31;
-  const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int n = blockIdx.x * ROWS + threadIdx.y;
   // the scale vector is a weight and the row list comes with the step's host copy: both are fetched
   // while the kernel before this one is still running
-  float wv[NC][8];
+  float4 wv[NV];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int h = (c * 32 + lane) * 8;
-    *reinterpret_cast<float4*>(wv[c]) = __ldg(reinterpret_cast<const float4*>(w + h));
-    *reinterpret_cast<float4*>(wv[c] + 4) = __ldg(reinterpret_cast<const float4*>(w + h + 4));
-  }
+  for (int c = 0; c < NV; ++c) wv[c] = __ldg(reinterpret_cast<const float4*>(w) + c * (WARPS * 32) + threadIdx.x);
   const int src_row = n < n_rows ? (rows ? __ldg(rows + n) : n) : 0;
   pdl_wait();
   if (n >= n_rows) return;
-  float* r = resid + (size_t)src_row * H;
-  const __nv_bfloat16* d = delta ? delta + (size_t)src_row * H : nullptr;
-  float x[NC][8];
-  uint4 dv[NC];
+  float* r = resid + (size_t)src_row * H + threadIdx.x * 4;
+  float4 x[NV], dv[NV];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int h = (c * 32 + lane) * 8;
-    *reinterpret_cast<float4*>(x[c]) = __ldcg(reinterpret_cast<const float4*>(r + h));
-    *reinterpret_cast<float4*>(x[c] + 4) = __ldcg(reinterpret_cast<const float4*>(r + h + 4));
-    if (d) dv[c] = __ldcg(reinterpret_cast<const uint4*>(d + h));
+  for (int c = 0; c < NV; ++c) x[c] = ld_four(r + c * STEP);
+  if (delta) {
+    const T* d = delta + (size_t)src_row * H + threadIdx.x * 4;
+#pragma unroll
+    for (int c = 0; c < NV; ++c) dv[c] = ld_four(d + c * STEP);
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      x[c].x += dv[c].x; x[c].y += dv[c].y; x[c].z += dv[c].z; x[c].w += dv[c].w;
+      if (!rows) st_four(r + c * STEP, x[c]);
+    }
   }
   float ss = 0.f;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int h = (c * 32 + lane) * 8;
-    if (d) {
-      float f[8];
-      bf16x8_to_f32(dv[c], f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[c][i] += f[i];
-      if (!rows) {
-        *reinterpret_cast<float4*>(r + h) = *reinterpret_cast<const float4*>(x[c]);
-        *reinterpret_cast<float4*>(r + h + 4) = *reinterpret_cast<const float4*>(x[c] + 4);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ss += x[c][i] * x[c][i];
-  }
+  for (int c = 0; c < NV; ++c) ss += (x[c].x * x[c].x + x[c].y * x[c].y) + (x[c].z * x[c].z + x[c].w * x[c].w);
   ss = warp_sum(ss);
-  const float rstd = rsqrtf(ss / (float)H + eps);
-  __nv_bfloat16* o = out + (size_t)n * H;
+  if constexpr (WARPS > 1) {
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = s_part[0];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int h = (c * 32 + lane) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[c][i] = x[c][i] * rstd * wv[c][i];
-    *reinterpret_cast<uint4*>(o + h) = f32_to_bf16x8(x[c]);
+    for (int i = 1; i < WARPS; ++i) ss += s_part[i];
   }
+  const float rstd = rsqrtf(ss / (float)H + eps);
+  T* o = out + (size_t)n * H + threadIdx.x * 4;
+#pragma unroll
+  for (int c = 0; c < NV; ++c)
+    st_four(o + c * STEP, make_float4(x[c].x * rstd * wv[c].x, x[c].y * rstd * wv[c].y, x[c].z * rstd * wv[c].z, x[c].w * rstd * wv[c].w));
 }
 
-template <int NC>
-static void launch_add_rmsnorm_warp(float* resid, const void* delta, const int* rows, const float* w, float eps, void* out,
-                                    int n_rows, cudaStream_t stream) {
-  const int warps = 4;
-  qe_launch(add_rmsnorm_bf16_warp_kernel<NC>, dim3((n_rows + warps - 1) / warps), dim3(warps * 32), 0, stream, resid,
-            (const __nv_bfloat16*)delta, rows, w, eps, (__nv_bfloat16*)out, n_rows);
+template <typename T, int NV, int WARPS>
+static void launch_add_rmsnorm_row(float* resid, const void* delta, const int* rows, const float* w, float eps, void* out,
+                                   int n_rows, cudaStream_t stream) {
+  constexpr int ROWS = WARPS == 1 ? 4 : 1;
+  qe_launch(add_rmsnorm_row_kernel<T, NV, WARPS, ROWS>, dim3((n_rows + ROWS - 1) / ROWS), dim3(WARPS * 32, ROWS), 0, stream, resid,
+            (const T*)delta, rows, w, eps, (T*)out, n_rows);
+}
+// Widths of the models: four warps a row up to 4 096, two where the width is an odd multiple of 256 (at 256 a warp, and four
+// rows a CTA: with a CTA of two warps 4 096 rows took 4.8 us, 3.8 with a warp a row).  False: not one of them.
+template <typename T>
+static bool launch_add_rmsnorm_rows(float* resid, const void* delta, const int* rows, const float* w, float eps, void* out,
+                                    int n_rows, int H, cudaStream_t stream) {
+#define NORM_ROW(NV, WARPS) case NV * WARPS * 128: launch_add_rmsnorm_row<T, NV, WARPS>(resid, delta, rows, w, eps, out, n_rows, stream); return true
+  switch (H) {
+    NORM_ROW(1, 4); NORM_ROW(2, 4); NORM_ROW(3, 4); NORM_ROW(4, 4); NORM_ROW(5, 4); NORM_ROW(6, 4); NORM_ROW(7, 4); NORM_ROW(8, 4);
+    NORM_ROW(2, 1); NORM_ROW(3, 2); NORM_ROW(5, 2); NORM_ROW(7, 2);
+  }
+#undef NORM_ROW
+  return false;
 }
 
 extern "C" int qe_add_rmsnorm(float* resid, const void* delta, const int* rows, const float* w,
@@ -233,23 +250,18 @@ extern "C" int qe_add_rmsnorm(float* resid, const void* delta, const int* rows, 
   const int threads = H >= 1024 ? 256 : (H >= 256 ? 128 : 64);
   if (dtype == QE_DTYPE_BF16 && H % 8 == 0 &&
       (((uintptr_t)resid | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-    if (H % 256 == 0 && H <= 2048) {
-      switch (H / 256) {
-        case 1: launch_add_rmsnorm_warp<1>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        case 2: launch_add_rmsnorm_warp<2>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        case 3: launch_add_rmsnorm_warp<3>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        case 4: launch_add_rmsnorm_warp<4>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        case 5: launch_add_rmsnorm_warp<5>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        case 6: launch_add_rmsnorm_warp<6>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        case 7: launch_add_rmsnorm_warp<7>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-        default: launch_add_rmsnorm_warp<8>(resid, delta, rows, w, eps, out, n_rows, stream); break;
-      }
+    if (launch_add_rmsnorm_rows<__nv_bfloat16>(resid, delta, rows, w, eps, out, n_rows, H, stream)) {
       QE_CHECK_LAUNCH("add_rmsnorm");
       return 0;
     }
     const int vthreads = H >= 2048 ? 256 : 128;
     qe_launch(add_rmsnorm_bf16x8_kernel, dim3(n_rows), dim3(vthreads), 0, stream, resid, (const __nv_bfloat16*)delta,
               rows, w, eps, (__nv_bfloat16*)out, H);
+    QE_CHECK_LAUNCH("add_rmsnorm");
+    return 0;
+  }
+  if (dtype == QE_DTYPE_F32 && (((uintptr_t)resid | (uintptr_t)delta | (uintptr_t)w | (uintptr_t)out) & 15) == 0 &&
+      launch_add_rmsnorm_rows<float>(resid, delta, rows, w, eps, out, n_rows, H, stream)) {
     QE_CHECK_LAUNCH("add_rmsnorm");
     return 0;
   }

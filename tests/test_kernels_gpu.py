@@ -1252,3 +1252,29 @@ def test_a_few_tokens_of_every_request_in_clusters(Hq, Hkv, q_lens, ctx_lens, pa
     got = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, 0, ops.paged_attention, DEV)
     assert ops.last_attention_kernel == "decode_attention_mma"
     _close(got, want, dtype)
+
+
+@pytest.mark.parametrize("T", [1, 3, 40])
+@pytest.mark.parametrize("H", [256, 512, 768, 1024, 1280, 1536, 1792, 2048, 2560, 3072, 3584, 4096])
+@pytest.mark.parametrize("with_delta", [False, True])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_add_rmsnorm_with_the_row_in_registers(T, H, with_delta, dtype):
+    """Widths of 128 channels a warp and piece: four warps a row, two where the width is an odd multiple of 256, one at 256."""
+    resid, w, eps = _randn((T, H), torch.float32, 81, 2.0), 1 + 0.3 * _randn((H,), torch.float32, 82), 1e-5
+    delta = _randn((T, H), dtype, 83) if with_delta else None
+    rows = torch.tensor([T - 1, 0], dtype=torch.int32)
+    for chosen in (None, rows):
+        total = resid.double() + (delta.double() if with_delta else 0.0)
+        pick = total if chosen is None else total[chosen.long()]
+        want = (pick * torch.rsqrt((pick * pick).mean(dim=1, keepdim=True) + eps) * w.double()).float()
+        stream, got = resid.to(DEV), torch.empty(want.shape, dtype=dtype, device=DEV)
+        d = delta.to(DEV) if with_delta else None
+        if chosen is None:
+            ops.add_rmsnorm(stream, d, w.to(DEV), eps, got)
+        else:
+            ops.add_rmsnorm_rows(stream, d, rows.to(DEV), w.to(DEV), eps, got)
+        _close(stream, total.float() if chosen is None and with_delta else resid, torch.float32, tol32=1e-6)
+        # bfloat16: a value is rounded once (7 stored bits of mantissa): half a unit in the last place is at most 2^-8 of it, and
+        # what float32 adds is a part in 10^6
+        part = 2.0 ** -8 * 1.01 if dtype == torch.bfloat16 else 2e-6
+        assert ((got.cpu().float() - want).abs() <= want.abs() * part + 1e-6).all()
