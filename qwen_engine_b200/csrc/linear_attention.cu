@@ -430,8 +430,232 @@ gla_scan_kernel(GlaArgs A) {
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// the scan of prompt portions whose rows come in whole pieces of 16 bytes
+// ---------------------------------------------------------------------------------------------------------
+// The arithmetic and the order of every sum are gla_scan_kernel's (the bits are the same).  What bounds that kernel is its
+// producers: they convert and scale what they stage, some 30 instructions a token and warp, one after the other (200
+// cycles a token whatever the computing threads do).  Here chunks come as they are stored, by 16-byte asynchronous copies
+// into a ring of three, which the computing threads ask for themselves (a few instructions a token), and each thread
+// unpacks what it reads.  The pieces of a row lie so that the L threads of a column read neighbouring 16 bytes.
+#define GLA_RING 3
+
+// DC channels out of the pieces that hold them
+template <int DC> __device__ __forceinline__ void gla_unpack(const uint4 (&r)[DC / 8], float (&f)[DC], __nv_bfloat16) {
+#pragma unroll
+  for (int i = 0; i < DC / 8; ++i) {
+    const uint32_t w[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+#pragma unroll
+    for (int x = 0; x < 4; ++x) { f[8 * i + 2 * x] = __uint_as_float(w[x] << 16); f[8 * i + 2 * x + 1] = __uint_as_float(w[x] & 0xffff0000u); }
+  }
+}
+template <int DC> __device__ __forceinline__ void gla_unpack(const uint4 (&r)[DC / 4], float (&f)[DC], float) {
+#pragma unroll
+  for (int i = 0; i < DC / 4; ++i) {
+    f[4 * i] = __uint_as_float(r[i].x); f[4 * i + 1] = __uint_as_float(r[i].y);
+    f[4 * i + 2] = __uint_as_float(r[i].z); f[4 * i + 3] = __uint_as_float(r[i].w);
+  }
+}
+// a pair of channels of one column through a token: s = a s + k v, acc = q s + acc (a rounded product, then fused
+// multiply-adds, two an instruction)
+__device__ __forceinline__ void gla_pair(float2& s, float2& acc, float ax, float ay, float kx, float ky, float qx, float qy, float v) {
+  asm("{\n\t.reg .b64 a, k, q, v, s, c;\n\t"
+      "mov.b64 a, {%4, %5};\n\tmov.b64 k, {%6, %7};\n\tmov.b64 q, {%8, %9};\n\tmov.b64 v, {%10, %10};\n\t"
+      "mov.b64 s, {%0, %1};\n\tmov.b64 c, {%2, %3};\n\t"
+      "mul.rn.f32x2 k, k, v;\n\tfma.rn.f32x2 s, a, s, k;\n\tfma.rn.f32x2 c, q, s, c;\n\t"
+      "mov.b64 {%0, %1}, s;\n\tmov.b64 {%2, %3}, c;\n\t}\n"
+      : "+f"(s.x), "+f"(s.y), "+f"(acc.x), "+f"(acc.y)
+      : "f"(ax), "f"(ay), "f"(kx), "f"(ky), "f"(qx), "f"(qy), "f"(v));
+}
+
 template <typename T, int DC>
-static int gla_launch(const GlaArgs& A, int R, cudaStream_t stream, size_t smem) {
+__global__ void __launch_bounds__(GLA_MAX_COMPUTE)
+gla_stream_kernel(GlaArgs A) {
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  constexpr int VEC = 16 / (int)sizeof(T), PT = DC / VEC, PA = DC / 4;       // pieces of a thread's channels: q, k; alpha
+  const int req = blockIdx.x, head = blockIdx.y, VT = A.VT, j0 = blockIdx.z * VT;
+  const int dk = A.dk, dv = A.dv, L = A.L, H = A.H, chunk = A.chunk;
+  const int tid = threadIdx.x, n_thr = blockDim.x;
+  const int j = j0 + tid / L, l = tid % L;
+  const bool owns = j < dv;
+  const unsigned col_mask = L >= 32 ? 0xffffffffu : (((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1)));
+  // a stage: q rows, k rows, alpha rows (float32), v rows
+  const int q_bytes = chunk * dk * (int)sizeof(T), a_bytes = A.head_decay ? 0 : chunk * dk * 4, v_bytes = chunk * VT * (int)sizeof(T);
+  const int stage_bytes = 2 * q_bytes + a_bytes + v_bytes;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row0 = A.cu_q[req];
+  const int n = A.cu_q[req + 1] - row0;
+  if (n <= 0) return;
+  const int ctx = A.ctx_lens[req], slot = A.slot_ids[req];
+  const int n_chunks = (n + chunk - 1) / chunk;
+  const T* q = (const T*)A.q + (size_t)head * dk;
+  const T* k = (const T*)A.k + (size_t)head * dk;
+  const T* v = (const T*)A.v + (size_t)head * dv + j0;
+  const float* al = A.alpha + (size_t)head * dk;
+  const float hd = A.head_decay ? A.head_decay[head] : 0.f;
+  // pieces a row (powers of two: the launcher's rule), and where piece x = l * (pieces a thread) + i lies: at i * L + l
+  const int sh_q = __ffs(dk / VEC) - 1, sh_a = __ffs(dk / 4) - 1, sh_v = __ffs(VT / VEC) - 1;
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gs_smem);
+  auto copy = [&](uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(dst), "l"(src) : "memory");
+  };
+  auto issue = [&](int ch) {
+    if (ch < n_chunks) {
+      const int t_first = ch * chunk, rows = min(chunk, n - t_first);
+      const size_t base = (size_t)(row0 + t_first);
+      const uint32_t st = ring + (uint32_t)(ch % GLA_RING) * stage_bytes;
+      for (int e = tid; e < rows << sh_q; e += n_thr) {
+        const int t = e >> sh_q, x = e & ((1 << sh_q) - 1);
+        const uint32_t at = st + (uint32_t)((t << sh_q) + (x % PT) * L + x / PT) * 16;
+        copy(at, q + (base + t) * A.ldq + x * VEC);
+        copy(at + q_bytes, k + (base + t) * A.ldk + x * VEC);
+      }
+      if (!A.head_decay)
+        for (int e = tid; e < rows << sh_a; e += n_thr) {
+          const int t = e >> sh_a, x = e & ((1 << sh_a) - 1);
+          copy(st + 2 * q_bytes + (uint32_t)((t << sh_a) + (x % PA) * L + x / PA) * 16, al + (base + t) * ((size_t)H * dk) + x * 4);
+        }
+      for (int e = tid; e < rows << sh_v; e += n_thr) {
+        const int t = e >> sh_v, x = e & ((1 << sh_v) - 1);
+        if (j0 + x * VEC < dv) copy(st + 2 * q_bytes + a_bytes + (uint32_t)e * 16, v + (base + t) * A.ldv + x * VEC);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  issue(0);
+  issue(1);
+
+  float* st = A.state + (((size_t)slot * H + head) * dv + (owns ? j : 0)) * dk + l * DC;
+  float2 s[DC / 2];
+#pragma unroll
+  for (int i = 0; i < DC / 4; ++i) {
+    const float4 x = owns && ctx > 0 ? *reinterpret_cast<const float4*>(st + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    s[2 * i] = make_float2(x.x, x.y); s[2 * i + 1] = make_float2(x.z, x.w);
+  }
+  const float q_scale = A.q_scale;
+  const size_t o_ld = (size_t)H * dv;
+  for (int ch = 0; ch < n_chunks; ++ch) {
+    asm volatile("cp.async.wait_group %0;\n" :: "n"(GLA_RING - 2) : "memory");
+    __syncthreads();                                  // the chunk has landed, and nobody reads the stage that is filled next
+    issue(ch + GLA_RING - 1);
+    const int rows = min(chunk, n - ch * chunk);
+    const unsigned char* base = gs_smem + (size_t)(ch % GLA_RING) * stage_bytes;
+    const T* qp = reinterpret_cast<const T*>(base) + l * VEC;
+    const T* kp = reinterpret_cast<const T*>(base + q_bytes) + l * VEC;
+    const float* ap = reinterpret_cast<const float*>(base + 2 * q_bytes) + l * 4;
+    const T* vp = reinterpret_cast<const T*>(base + 2 * q_bytes + a_bytes) + (j - j0);
+    float* o = A.out + (size_t)(row0 + ch * chunk) * o_ld + (size_t)head * dv + j;
+    struct Token { uint4 q[PT], k[PT], a[PA]; T v; };
+    auto load = [&](int t, Token& x) {
+#pragma unroll
+      for (int i = 0; i < PT; ++i) {
+        x.q[i] = *reinterpret_cast<const uint4*>(qp + (size_t)t * dk + i * L * VEC);
+        x.k[i] = *reinterpret_cast<const uint4*>(kp + (size_t)t * dk + i * L * VEC);
+      }
+      if (!A.head_decay) {
+#pragma unroll
+        for (int i = 0; i < PA; ++i) x.a[i] = *reinterpret_cast<const uint4*>(ap + (size_t)t * dk + i * L * 4);
+      }
+      x.v = vp[(size_t)t * VT];
+    };
+    auto step = [&](const Token& x) -> float {        // (sums in gla_scan_kernel's order)
+      float qf[DC], kf[DC], af[DC];
+      gla_unpack<DC>(x.q, qf, T());
+      gla_unpack<DC>(x.k, kf, T());
+      if (A.head_decay) {
+#pragma unroll
+        for (int i = 0; i < DC; ++i) af[i] = hd;
+      } else {
+        gla_unpack<DC>(x.a, af, 0.f);
+      }
+      const float vj = to_f32(x.v);
+      float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < DC; i += 2)
+        gla_pair(s[i / 2], acc, af[i], af[i + 1], kf[i], kf[i + 1], qf[i] * q_scale, qf[i + 1] * q_scale, vj);
+      return acc.x + acc.y;
+    };
+    Token ahead;                                      // the next token's operands are on their way while one is worked on
+    load(0, ahead);
+    int t0 = 0;
+    for (; t0 + 8 <= rows; t0 += 8) {                 // eight tokens a turn: see gla_scan_kernel
+      float acc[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const Token now = ahead;
+        load(min(t0 + u + 1, rows - 1), ahead);
+        acc[u] = step(now);
+      }
+      int mine = 0, held = 8;
+#pragma unroll
+      for (int off = 1; off < 8; off <<= 1) {
+        if (L > off) {
+          const bool up = l & off;
+          const int half = 4 / off;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (i >= half) continue;
+            const float give = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(col_mask, give, off);
+          }
+          mine += up ? half : 0;
+          held = half;
+        }
+      }
+      for (int off = 8; off < L; off <<= 1) acc[0] += __shfl_xor_sync(col_mask, acc[0], off);
+      if (l < 8 && owns) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) if (i < held) o[(size_t)(t0 + mine + i) * o_ld] = acc[i];
+      }
+    }
+    for (; t0 < rows; ++t0) {
+      const Token now = ahead;
+      load(min(t0 + 1, rows - 1), ahead);
+      float acc = step(now);
+      for (int off = 1; off < L; off <<= 1) acc += __shfl_xor_sync(col_mask, acc, off);
+      if (l == 0 && owns) o[(size_t)t0 * o_ld] = acc;
+    }
+  }
+  if (owns && A.write_state) {
+#pragma unroll
+    for (int i = 0; i < DC / 4; ++i) *reinterpret_cast<float4*>(st + 4 * i) = make_float4(s[2 * i].x, s[2 * i].y, s[2 * i + 1].x, s[2 * i + 1].y);
+  }
+}
+
+// Whether gla_stream_kernel serves: rows in whole pieces of 16 bytes, every thread's channels whole pieces of the
+// head, and powers of two of them; and not a long prompt alone.  Its warps have more to do for a token, and where an SM holds
+// one CTA of two warps their latency counts, while gla_scan_kernel's CTAs find room one to an SM and wait for a second round beyond.
+// Measured on a B200, 64 key and 128 value channels in bfloat16, 8 heads (gla_scan_kernel / gla_stream_kernel): 8 requests of 256 tokens
+// 131.8 / 66.8 us, 32 of 64 166 / 61, 4 of 512 on average 236 / 121, one of 9 5.8 / 3.8, one of 40 10.7 / 7.9, but one of 2 048 202 / 266 (128 key
+// channels, 1 024 tokens 199 / 222); 256 and 512 key channels, one of 512 tokens 293 / 270 and 559 / 296.
+template <typename T, int DC>
+static bool gla_streams(const GlaArgs& A, int R, int max_q_len) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  if ((long)R * A.H * ((A.dv + A.VT - 1) / A.VT) <= 148 && max_q_len > 128 && A.dk < 256) return false;
+  return DC >= VEC && !A.single && A.vec && A.da == nullptr && A.dk == A.L * DC && A.VT % VEC == 0 && ((A.VT / VEC) & (A.VT / VEC - 1)) == 0 && (A.VT * A.L) % 32 == 0;
+}
+template <typename T, int DC>
+static int gla_stream_launch(GlaArgs A, int R, int max_q_len, cudaStream_t stream) {
+  const size_t token = (size_t)A.dk * (2 * sizeof(T) + (A.head_decay ? 0 : 4)) + (size_t)A.VT * sizeof(T);
+  A.chunk = max_q_len < 32 ? max_q_len : 32;
+  while (A.chunk > 8 && GLA_RING * A.chunk * token > 72 * 1024) A.chunk = (A.chunk / 2 + 7) / 8 * 8;
+  const size_t smem = GLA_RING * A.chunk * token;
+  static const cudaError_t configured = cudaFuncSetAttribute(gla_stream_kernel<T, DC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  if (configured != cudaSuccess) QE_REFUSE("linear_attention_scan: shared memory: %s", cudaGetErrorString(configured));
+  if (smem > 220 * 1024) return -1;
+  qe_launch(gla_stream_kernel<T, DC>, dim3(R, A.H, (A.dv + A.VT - 1) / A.VT), dim3(A.VT * A.L), smem, stream, A);
+  QE_CHECK_LAUNCH("linear_attention_scan");
+  return 0;
+}
+
+template <typename T, int DC>
+static int gla_launch(const GlaArgs& A, int R, int max_q_len, cudaStream_t stream, size_t smem) {
+  if constexpr (DC >= 16 / (int)sizeof(T))
+    if (gla_streams<T, DC>(A, R, max_q_len)) {
+      const int rc = gla_stream_launch<T, DC>(A, R, max_q_len, stream);
+      if (rc >= 0) return rc;                         // (below: its ring does not fit)
+    }
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gla_scan_kernel<T, DC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
@@ -507,7 +731,7 @@ extern "C" int qe_linear_attention_scan(const void* q, const void* k, const void
           ldv % vec_n == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)alpha) & 15) == 0;
   const size_t smem = (size_t)2 * chunk * tok_w * sizeof(float);
   if (smem > 96 * 1024) QE_REFUSE("linear_attention_scan: key size %d needs %zu bytes of shared memory", dk, smem);
-#define GLA_CASE(TT, DCC) return gla_launch<TT, DCC>(A, R, stream, smem)
+#define GLA_CASE(TT, DCC) return gla_launch<TT, DCC>(A, R, max_q_len, stream, smem)
   if (dtype == QE_DTYPE_F32) {
     switch (DC) { case 4: GLA_CASE(float, 4); case 8: GLA_CASE(float, 8); case 16: GLA_CASE(float, 16); default: GLA_CASE(float, 32); }
   } else if (dtype == QE_DTYPE_BF16) {

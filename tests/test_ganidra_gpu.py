@@ -429,3 +429,29 @@ def test_the_command_line_replays_a_trace(folders, tmp_path):
     last = torch.frombuffer(bytearray((out / "2.f32").read_bytes()), dtype=F32).reshape(-1, V)
     gh.assert_close_rows(first, want[[0, 20]], F32, "step 0")
     gh.assert_close_rows(last, torch.stack([want[29], want[3]]), F32, "step 2")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("H,dk,dv", [(2, 32, 16), (8, 64, 128), (1, 64, 40), (3, 128, 128), (2, 256, 24), (1, 512, 8), (1, 1024, 8), (2, 16, 32)])
+@pytest.mark.parametrize("lens", [[2], [31, 1, 33], [32, 64, 9], [200, 1, 7, 96]])
+@pytest.mark.parametrize("constant", [False, True])
+def test_scan_of_whole_pieces_gives_the_general_paths_bits(ops, dtype, H, dk, dv, lens, constant):
+    """Rows in whole pieces of 16 bytes go through a ring of asynchronous copies (chunks of 8 to 32 tokens, their edges, tails of a turn of
+    eight, requests of one token among others, columns behind the last): the same bits, outputs and states, as rows that
+    start an element off, which the general kernel stages itself; a decay per channel, or one per head."""
+    T, width = sum(lens), 2 * H * dk + H * dv
+    g = torch.Generator().manual_seed(dk + dv + T)
+    rows = torch.randn(T, width, generator=g).to(dtype).to(DEV)
+    off = torch.empty(T, width + 9, dtype=dtype, device=DEV)[:, 1:1 + width]
+    off.copy_(rows)
+    alpha = (torch.rand(T, H * dk, generator=g) * 0.5 + 0.5).to(DEV)
+    heads = (torch.rand(H, generator=g) * 0.5 + 0.5).to(DEV) if constant else None
+    ctx = _ctx(lens, [r % 2 for r in range(len(lens))], list(range(len(lens))))       # (every other request has a context)
+    got = []
+    for x in (rows, off):
+        state = torch.randn(len(lens), H, dv, dk, generator=torch.Generator().manual_seed(3)).to(DEV)
+        out = torch.zeros(T, H * dv, dtype=F32, device=DEV)
+        ops.linear_attention_scan(x[:, :H * dk], x[:, H * dk:2 * H * dk], x[:, 2 * H * dk:], None if constant else alpha, state, ctx, out,
+                                  dk ** -0.5, H, dk, dv, head_decay=heads)
+        got.append((out, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
