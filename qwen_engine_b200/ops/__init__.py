@@ -1273,14 +1273,15 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
                 keys = attended_keys([q_lens[r] for r in rest], [ctx_lens[r] for r in rest], window)
                 items_in_all = parts_for_lengths(geo, keys, max(-(-k // min(-(-k // FLASH_SPLIT), at_most)) for k in keys),
                                                  max(q_lens[r] for r in rest) * G)
-        most_parts = max(1, FLASH_TARGET_CTAS // max(1, base))
+        every = None                                    # the number of parts of every request, where it is the same for all
         if (uniform_splits is None and rest and len(rest) == len(q_lens) and DECODE_ATTENTION_MMA and DECODE_ATTENTION_MMA_WIDE and D == 128
                 and geometry_planes(geo) >= 2 and base <= TC_TARGET_CTAS and max(q_lens) * G <= 16):
-            # a few tokens of every request, nothing else: CTAs of 8 warps, one per SM, and parts that form clusters, as for decoded
-            # tokens (7 requests of one token and one of three behind 1 300 keys, 12 rows: 24.9 us in 4 parts of 4 warps, of
-            # which two with their in-boxes do not fit an SM, 12.9 in 2 parts of 8)
-            span = max(attended_keys(q_lens, ctx_lens, window))
-            most_parts = _cluster_parts(max(1, min(TC_TARGET_CTAS // base, -(-span // FLASH_SPLIT))), base, span)
+            # a few tokens of every request, nothing else
+            parts = few_token_parts(geo, attended_keys(q_lens, ctx_lens, window), max(q_lens) * G)
+            if isinstance(parts, TotalParts):
+                items_in_all = parts
+            else:
+                every = parts
         if items_in_all is not None:
             dealt = items_in_all.shares
             if dealt is None:
@@ -1300,11 +1301,13 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
                 splits = shares[r]
             elif uniform_splits is not None:
                 splits = uniform_splits[geo]
+            elif every is not None:
+                splits = every
             else:
                 lo = (max(0, c - window + 1) // FLASH_BN) * FLASH_BN if window else 0
                 splits = 1
                 if n <= tpt and base < FLASH_TARGET_CTAS and total - lo > FLASH_SPLIT:
-                    splits = min(-(-(total - lo) // FLASH_SPLIT), most_parts)
+                    splits = min(-(-(total - lo) // FLASH_SPLIT), max(1, FLASH_TARGET_CTAS // base))
             if splits > 1:
                 for sp in range(splits):
                     item = [r, 0, 0, 0, n_parts + sp, splits, sp, row0, n, c, 0, 0]
@@ -1347,6 +1350,7 @@ def plan_attention(q_lens: list[int], ctx_lens: list[int], page_size: int,
 
 
 DECODE_CLUSTER4_MAX_SPAN = 4096   # keys up to which 4 parts in a cluster are preferred to more parts merged through memory
+DECODE_CLUSTER4_MAX_CTAS = 128    # CTAs of 8 warps in clusters of 4 that find room at once
 
 
 def _cluster_parts(parts: int, ctas: int, span: int) -> int:
@@ -1365,6 +1369,46 @@ def _cluster_parts(parts: int, ctas: int, span: int) -> int:
     if few or (parts == 8 and span > DECODE_CLUSTER4_MAX_SPAN):
         return 8
     return 4 if span <= DECODE_CLUSTER4_MAX_SPAN else parts
+
+
+def few_token_parts(geo, keys: list[int], rows: int):
+    """How the contexts of a step that brings a few tokens of every request and nothing else (``rows``: the most rows of one, at
+    most 16; ``keys``: what each attends to) are cut: a number of parts of every request, which form clusters where it is 2, 4 or
+    8, or the work items of all requests, dealt out by length (``TotalParts``).  The items are CTAs of 8 warps, one per SM, as
+    far as they fit.
+
+    The longest part sets the time: 0.0091 us a key.  Parts that meet in a cluster cost next to nothing; parts that are added up through memory
+    as much as 300 keys and 15 for each row, whichever requests they belong to.  So contexts of about equal lengths form
+    clusters, others get parts by their lengths, and where neither shortens the longest by more than that they stay whole, or
+    go to CTAs of 4 warps, two per SM, by ``parts_for_lengths``'s rule.  From five rows on 8 parts of less than a split each are
+    1.1 to 1.3 times as slow as 4 (16 / 8 heads, 4 tokens behind 600 and 1 700 keys 8.5, 9.8 us / 6.4, 8.1; 2 tokens 4.5, 5.7 / 4.8, 6.5), and 36 clusters of 4
+    do not all find room (16 / 2 heads, 18 requests of 1 300 keys 28.0 us, in clusters of 2 14.4).
+
+    Measured on a B200 (a chain of launches; every request in parts of 256 keys, as far as 296 CTAs go / at most as many parts
+    as the longest would get if all were like it / this rule), 16 / 8 heads, one request of 2 tokens, the others 1: 16 000 keys beside nine
+    requests of 200 54.9 / 146.6 / 23.4 us, beside five 29.5 / 79.6 / 19.0, ten of 150 to 2 045 15.0 / 20.1 / 11.9; ten of 8 tokens behind 2 000 31.1 /
+    26.8 / 26.7, five of 2 behind 4 000 19.4 / 24.0 / 18.8; one of 2 tokens behind 600, 1 400 and 3 000 6.9, 7.2, 8.8 / 6.8, 7.3, 7.0 / 4.8, 5.5,
+    7.0.  32 / 8 heads, seven of one token and one of three behind 1 300 26.2 / 13.1 / 13.1.  Over some 200 batches the times are 0.79
+    and 0.84 of the other two's; the few that lose, lose 4 to 9 % (18 requests of 4 000 keys whole 49.3 / 51.2 / 51.5), one 18 (one
+    request of 160 keys beside two of 1 200 and 1 700 with 16 rows 9.9 / 11.1 / 11.7)."""
+    base, n = geo[1] * value_blocks(geo), len(keys)
+    span = max(keys)
+    parts = _cluster_parts(max(1, min(TC_TARGET_CTAS // (n * base), -(-span // FLASH_SPLIT))), n * base, span)
+    if parts == 8 and span < 8 * FLASH_SPLIT and rows > 4:
+        parts = 4
+    if parts == 4 and n * base * 4 > DECODE_CLUSTER4_MAX_CTAS:
+        parts = 2
+    slots = TC_TARGET_CTAS // base
+    dealt = parts_by_length(keys, slots) if DECODE_PARTS_BY_LENGTH and n < slots else None
+    longest = max(-(-k // p) for k, p in zip(keys, dealt)) if dealt else span
+    cost = 300 + 15 * rows
+    if parts in (2, 4, 8) and -(-span // parts) <= longest + cost:
+        return parts
+    if longest + cost <= span:
+        total = TotalParts(sum(dealt))
+        total.shares = dealt
+        return total
+    return parts_for_lengths(geo, keys, -(-span // 2), rows) or 1
 
 
 def decode_splits(num_reqs: int, max_tokens: int, geometries, dtype: torch.dtype, ctx_lens: Optional[list] = None) -> dict:

@@ -230,3 +230,51 @@ def test_contexts_stay_whole_where_cutting_them_costs_more(heads, kv_heads, ctx)
 def test_contexts_are_cut_where_one_of_them_sets_the_time(heads, kv_heads, ctx):
     geo, bf = (heads, kv_heads, 128, 0), torch.bfloat16
     assert type(ops.decode_splits(len(ctx), -(-max(ctx) // 1024) * 1024, (geo,), bf, ctx)[geo]) is ops.TotalParts
+
+
+@pytest.mark.parametrize("heads,kv_heads,q_lens,ctx_lens,want", [
+    (16, 8, [2], [600], 4), (16, 8, [2], [1100], 8), (16, 8, [4], [1700], 4), (16, 8, [8], [1200], 4), (8, 8, [2], [1400], 8),     # 3, 5, 7 splits of
+    (16, 8, [2, 2], [700, 700], 4), (16, 8, [2], [3000], 8), (16, 2, [2] * 18, [1300] * 18, 2), (16, 8, [2] * 8, [330] * 8, 2),    # 256 keys: the next cluster
+    (16, 8, [2] * 10, [700] * 10, 1), (32, 8, [2] * 18, [2900] * 18, 1), (16, 8, [3], [200], 1),
+    (16, 8, [2] + [1] * 9, [16000] + [200] * 9, [9] + [1] * 9), (16, 8, [2] + [1] * 5, [16000] + [200] * 5, [13] + [1] * 5),
+    (16, 8, [1, 2, 1], [40, 3000, 700], [9, 2]), (16, 8, [2] * 5, [4000] * 5, [4, 4, 4, 3, 3]),
+])
+def test_a_few_tokens_of_every_request_are_cut_by_their_lengths(heads, kv_heads, q_lens, ctx_lens, want):
+    """Contexts of about equal lengths form clusters of exactly 2, 4 or 8 parts, whatever the number of splits; others have parts by
+    their lengths, as many CTAs of 8 warps as SMs in all."""
+    plan = ops.plan_attention(q_lens, ctx_lens, 16, ((heads, kv_heads, 128, 0),), torch.bfloat16)
+    info = plan["fa0_info"]
+    if isinstance(want, int):
+        assert info[4] == (want if want > 1 else 0) and info[0] == (want * len(q_lens) if want > 1 else 0)
+        return
+    parts = {i[0]: i[5] or 1 for i in _items(plan, "fa0_items")}
+    assert info[4] == 0 and info[0] == len(plan["fa0_items"]) // 12 <= ops.TC_TARGET_CTAS // kv_heads and plan["fa0_merge"] == []
+    assert sorted((n for n in parts.values()), reverse=True)[:len(want)] == want
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_a_few_tokens_of_every_request_leave_no_key_and_no_place_out(seed):
+    """Any batch of a few tokens of every request: each request's parts are there once, with places of their own in the scratch
+    memory, which holds no more than an item of every CTA."""
+    rng = random.Random(600 + seed)
+    geo = ((16, 8, 128, 0), (32, 8, 128, 0), (16, 2, 128, 700), (8, 8, 128, 0, True), (16, 4, 128, 0, False, 3), (40, 40, 128, 0))[seed % 6]
+    G, R = geo[0] // geo[1], rng.randint(1, 20)
+    q = [rng.choice([1, rng.randint(1, 16 // G)]) for _ in range(R)]
+    q[rng.randrange(R)] = rng.randint(2, 16 // G)
+    ctx = [rng.choice([0, 40, 256, rng.randint(1, 2000), rng.randint(1, 20000) if rng.random() < 0.2 else 500]) for _ in range(R)]
+    plan = ops.plan_attention(q, ctx, 16, (geo,), torch.bfloat16)
+    items, (n_parts, part_rows, small, most, same) = _items(plan, "fa0_items"), plan["fa0_info"]
+    held = [i for i in items if i[8]]
+    assert small == 1 and most == max(q) * G and (not n_parts or part_rows >= max(n for i, n in enumerate(q) if any(h[0] == i and h[4] >= 0 for h in held)) * G)
+    places = [i[4] for i in held if i[4] >= 0]
+    assert sorted(places) == sorted(set(places)) and max(places, default=-1) < max(1, n_parts)
+    for r in range(R):
+        mine = sorted((i for i in held if i[0] == r), key=lambda i: i[6])
+        assert all(i[7:10] == [sum(q[:r]), q[r], ctx[r]] for i in mine)
+        if len(mine) == 1 and mine[0][4] < 0:
+            assert mine[0][2:7] == [0, ctx[r] + q[r], -1, 0, 0]
+        else:
+            assert [i[4:7] for i in mine] == [[mine[0][4] + s, len(mine), s] for s in range(len(mine))]
+            assert not same or len(mine) == same
+    if same:
+        assert same in (2, 4, 8) and len(items) == n_parts == same * R and [i[0] for i in items] == [r for r in range(R) for _ in range(same)]

@@ -1254,6 +1254,25 @@ def test_a_few_tokens_of_every_request_in_clusters(Hq, Hkv, q_lens, ctx_lens, pa
     _close(got, want, dtype)
 
 
+@pytest.mark.parametrize("Hq,Hkv,q_lens,ctx_lens,window", [
+    (16, 8, [2] + [1] * 9, [6000] + [200] * 9, 0), (32, 8, [1, 4, 2], [9000, 300, 40], 0), (8, 8, [16, 1, 3], [90, 4000, 1], 0),
+    (16, 2, [2, 1, 1], [9000, 15, 700], 0), (16, 8, [2] + [1] * 5, [9000] + [350] * 5, 4000), (16, 8, [2] * 10, [2900] * 10, 0),
+])
+@pytest.mark.parametrize("options", [{}, {"sinks": True}, {"softcap": 20.0}, {"slopes": True}])
+def test_a_few_tokens_of_every_request_in_parts_by_length(Hq, Hkv, q_lens, ctx_lens, window, options):
+    """Long contexts among short ones, 2 to 16 rows a request: parts by length, which meet through memory."""
+    P, dtype = 16, torch.bfloat16
+    geo = (Hq, Hkv, 128, window) + ((True,) if "slopes" in options else ())
+    info = ops.plan_attention(q_lens, ctx_lens, P, (geo,), dtype)["fa0_info"]
+    assert info[0] > 1 and info[4] == 0 and info[3] == max(q_lens) * Hq // Hkv
+    options = {k: torch.linspace(0.01, 0.6, Hq) if v is True else v for k, v in options.items()}
+    case = _attention_case(dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, window, seed=88)
+    want = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, window, ref_ops.paged_attention, "cpu", **options)
+    got = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, **options)
+    assert ops.last_attention_kernel == "decode_attention_mma"
+    _close(got, want, dtype)
+
+
 @pytest.mark.parametrize("T", [1, 3, 40])
 @pytest.mark.parametrize("H", [256, 512, 768, 1024, 1280, 1536, 1792, 2048, 2560, 3072, 3584, 4096])
 @pytest.mark.parametrize("with_delta", [False, True])
