@@ -623,17 +623,42 @@ gla_stream_kernel(GlaArgs A) {
   }
 }
 
+// The tile of value channels of a CTA, for DC key channels a thread and L threads a column: a column's threads lie within one
+// warp (L divides 32); a tile fills up to 128 threads, and is narrower where few requests would leave SMs idle.
+static int gla_tile(int R, int H, int dv, int L) {
+  int VT = GLA_MAX_COMPUTE / L;
+  if (VT > dv) VT = dv;
+  while (VT > 8 && (long)R * H * ((dv + VT - 1) / VT) < 296 && VT * L > 64) VT = (VT + 1) / 2;
+  return VT;
+}
+
+// Whether gla_stream_kernel is the faster one for R requests of `tokens` tokens between them, the longest of max_q_len;
+// token_bytes: what a token and head brings of q, k and alpha.  Its warps have more to do for a token, so a long prompt's
+// chain takes 1.1 to 1.3 times as long, and up to twice where CTAs of one prompt share an SM; gla_scan_kernel's
+// CTAs find room one to an SM, so the other requests wait for their turn there, each of their tokens twice as dear
+// as the long prompt's (chunks that nobody staged ahead) and some 80 tokens' time more for a request.  The line lies where an
+// SM's work exceeds the longest chain by what that chain loses.  From 256 key channels on gla_scan_kernel is the slower one anyway.
+// Measured on a B200 (gla_scan_kernel / gla_stream_kernel), 64 key and 128 value channels in bfloat16, 8 heads: 8 requests of 256 tokens
+// 139 / 74 us, two of 512 119 / 76, 1 024 + 200 + 100 200 / 171, 512 beside 63 of one 176 / 113, one of 9 10.4 / 9.2, one of 100 23.5 / 22.5, but one of
+// 2 048 220 / 270, beside 3 of one 228 / 352, beside 15 262 / 330, 512 beside 3 82 / 96, 1 024 + 64 134 / 143; 16 heads, 2 048 beside 3
+// 257 / 509, 512 beside 15 148 / 113.  128 key channels: 4 heads, 700 + 500 + 300 225 / 177, 2 048 beside 15 508 / 582; 8 heads of 256 value
+// channels, 512 beside 15 217 / 203, in float32 231 / 277 (a larger part of the ring's copies: its own line).  float32, 8 heads of 64: 2 048
+// beside 15 333 / 423, 8 of 256 170 / 94.  256 and 512 key channels, one of 512 tokens: 315 / 242 and 614 / 272, in float32 367 / 193 and 716 / 262.
+static bool gla_stream_pays(int R, int max_q_len, long tokens, int H, int dk, int dv, int VT, int L, int token_bytes) {
+  const long ctas_each = (long)H * ((dv + VT - 1) / VT);
+  if (dk >= 256 || max_q_len <= 128) return true;
+  if (R * ctas_each <= 148) return false;
+  const double work = (double)(2 * tokens - max_q_len + 80L * (R - 1)) * (double)ctas_each / 148.0;
+  return work > (token_bytes > 1024 && VT * L > 64 ? 3.0 : 1.4) * max_q_len;
+}
+
 // Whether gla_stream_kernel serves: rows in whole pieces of 16 bytes, every thread's channels whole pieces of the
-// head, and powers of two of them; and not a long prompt alone.  Its warps have more to do for a token, and where an SM holds
-// one CTA of two warps their latency counts, while gla_scan_kernel's CTAs find room one to an SM and wait for a second round beyond.
-// Measured on a B200, 64 key and 128 value channels in bfloat16, 8 heads (gla_scan_kernel / gla_stream_kernel): 8 requests of 256 tokens
-// 131.8 / 66.8 us, 32 of 64 166 / 61, 4 of 512 on average 236 / 121, one of 9 5.8 / 3.8, one of 40 10.7 / 7.9, but one of 2 048 202 / 266 (128 key
-// channels, 1 024 tokens 199 / 222); 256 and 512 key channels, one of 512 tokens 293 / 270 and 559 / 296.
+// head, and powers of two of them, and where it pays.
 template <typename T, int DC>
-static bool gla_streams(const GlaArgs& A, int R, int max_q_len) {
+static bool gla_streams(const GlaArgs& A, int R, int max_q_len, long tokens) {
   constexpr int VEC = 16 / (int)sizeof(T);
-  if ((long)R * A.H * ((A.dv + A.VT - 1) / A.VT) <= 148 && max_q_len > 128 && A.dk < 256) return false;
-  return DC >= VEC && !A.single && A.vec && A.da == nullptr && A.dk == A.L * DC && A.VT % VEC == 0 && ((A.VT / VEC) & (A.VT / VEC - 1)) == 0 && (A.VT * A.L) % 32 == 0;
+  return DC >= VEC && !A.single && A.vec && A.da == nullptr && A.dk == A.L * DC && A.VT % VEC == 0 && ((A.VT / VEC) & (A.VT / VEC - 1)) == 0 && (A.VT * A.L) % 32 == 0 &&
+         gla_stream_pays(R, max_q_len, tokens, A.H, A.dk, A.dv, A.VT, A.L, A.dk * (2 * (int)sizeof(T) + (A.head_decay ? 0 : 4)));
 }
 template <typename T, int DC>
 static int gla_stream_launch(GlaArgs A, int R, int max_q_len, cudaStream_t stream) {
@@ -650,9 +675,9 @@ static int gla_stream_launch(GlaArgs A, int R, int max_q_len, cudaStream_t strea
 }
 
 template <typename T, int DC>
-static int gla_launch(const GlaArgs& A, int R, int max_q_len, cudaStream_t stream, size_t smem) {
+static int gla_launch(const GlaArgs& A, int R, int max_q_len, long tokens, cudaStream_t stream, size_t smem) {
   if constexpr (DC >= 16 / (int)sizeof(T))
-    if (gla_streams<T, DC>(A, R, max_q_len)) {
+    if (gla_streams<T, DC>(A, R, max_q_len, tokens)) {
       const int rc = gla_stream_launch<T, DC>(A, R, max_q_len, stream);
       if (rc >= 0) return rc;                         // (below: its ring does not fit)
     }
@@ -672,6 +697,9 @@ static int gla_launch(const GlaArgs& A, int R, int max_q_len, cudaStream_t strea
   return 0;
 }
 
+// Whether a head and a tile of its value channels are whole pieces of vec_n elements.
+static bool gla_pieces(int vec_n, int dk, int dv, int VT) { return dk % vec_n == 0 && dk % 4 == 0 && VT % vec_n == 0 && dv % vec_n == 0; }
+
 // How the key channels of a head are dealt to threads: DC channels a thread, L threads a column.
 static void gla_shape(int dk, int* DC, int* L) {
   int dc = dk <= 16 ? 4 : dk <= 64 ? 8 : dk <= 128 ? 16 : 32;
@@ -680,11 +708,34 @@ static void gla_shape(int dk, int* DC, int* L) {
   *DC = dc; *L = l;
 }
 
+// Whether gla_stream_kernel takes a step of R requests (1) or gla_scan_kernel (0), for q, k, v and a decay per channel
+// whose rows are whole pieces of 16 bytes.
+template <typename T>
+static bool gla_streams_shape(int R, int max_q_len, int tokens, int H, int dk, int dv) {
+  GlaArgs A{};
+  int DC;
+  gla_shape(dk, &DC, &A.L);
+  A.H = H; A.dk = dk; A.dv = dv; A.single = max_q_len <= 1;
+  A.VT = gla_tile(R, H, dv, A.L);
+  A.vec = gla_pieces(16 / (int)sizeof(T), dk, dv, A.VT);
+  switch (DC) {
+    case 4: return gla_streams<T, 4>(A, R, max_q_len, tokens);
+    case 8: return gla_streams<T, 8>(A, R, max_q_len, tokens);
+    case 16: return gla_streams<T, 16>(A, R, max_q_len, tokens);
+    default: return gla_streams<T, 32>(A, R, max_q_len, tokens);
+  }
+}
+extern "C" int qe_linear_attention_scan_streams(int R, int max_q_len, int tokens, int H, int dk, int dv, int dtype) {
+  if (R < 1 || H < 1 || dk < 1 || dk > 1024 || dv < 1) return 0;
+  return dtype == QE_DTYPE_F32 ? gla_streams_shape<float>(R, max_q_len, tokens, H, dk, dv) : gla_streams_shape<__nv_bfloat16>(R, max_q_len, tokens, H, dk, dv);
+}
+
 // alpha null (steps of single tokens only): the decay comes from decay_a [T, rank] (rows of lda elements), decay_w
 // [H dk, rank] in the type of q, decay_bias float32 [H dk] and tau, as qe_channel_decay computes it.
+// tokens: of all requests, max_q_len of the longest; they choose between two kernels that give the same bits.
 extern "C" int qe_linear_attention_scan(const void* q, const void* k, const void* v, long ldq, long ldk, long ldv,
                                         const float* alpha, float* state, const int* cu_q, const int* ctx_lens,
-                                        const int* slot_ids, float* out, float q_scale, int R, int max_q_len, int H,
+                                        const int* slot_ids, float* out, float q_scale, int R, int max_q_len, int tokens, int H,
                                         int dk, int dv, int write_state, int dtype, const void* decay_a, long lda,
                                         const void* decay_w, const float* decay_bias, float tau, int rank,
                                         const float* head_decay, cudaStream_t stream) {
@@ -704,11 +755,7 @@ extern "C" int qe_linear_attention_scan(const void* q, const void* k, const void
   A.head_decay = head_decay;
   if (head_decay) decay_a = nullptr;
   A.da = alpha ? nullptr : decay_a; A.lda = lda; A.dw = decay_w; A.dbias = decay_bias; A.inv_tau = (alpha || head_decay) ? 0.f : 1.f / tau; A.R = rank;
-  // a column's threads lie within one warp (L divides 32); a tile of value channels fills up to 256 threads,
-  // and is narrower where few requests would leave SMs idle
-  int VT = GLA_MAX_COMPUTE / L;
-  if (VT > dv) VT = dv;
-  while (VT > 8 && (long)R * H * ((dv + VT - 1) / VT) < 296 && VT * L > 64) VT = (VT + 1) / 2;
+  const int VT = gla_tile(R, H, dv, L);
   A.VT = VT;
   const int row_w = L * DC + ((L * DC) / DC) * 4;
   const int tok_w = 3 * row_w + ((VT + 3) & ~3);
@@ -727,11 +774,11 @@ extern "C" int qe_linear_attention_scan(const void* q, const void* k, const void
   const int vec_n = dtype == QE_DTYPE_F32 ? 4 : 8;
   const int per_tok_pieces = 2 * (dk / vec_n) + dk / 4 + VT / vec_n;
   A.fast = chunk * per_tok_pieces <= 8 * GLA_PRODUCERS;
-  A.vec = dk % vec_n == 0 && dk % 4 == 0 && VT % vec_n == 0 && dv % vec_n == 0 && ldq % vec_n == 0 && ldk % vec_n == 0 &&
+  A.vec = gla_pieces(vec_n, dk, dv, VT) && ldq % vec_n == 0 && ldk % vec_n == 0 &&
           ldv % vec_n == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)alpha) & 15) == 0;
   const size_t smem = (size_t)2 * chunk * tok_w * sizeof(float);
   if (smem > 96 * 1024) QE_REFUSE("linear_attention_scan: key size %d needs %zu bytes of shared memory", dk, smem);
-#define GLA_CASE(TT, DCC) return gla_launch<TT, DCC>(A, R, max_q_len, stream, smem)
+#define GLA_CASE(TT, DCC) return gla_launch<TT, DCC>(A, R, max_q_len, tokens, stream, smem)
   if (dtype == QE_DTYPE_F32) {
     switch (DC) { case 4: GLA_CASE(float, 4); case 8: GLA_CASE(float, 8); case 16: GLA_CASE(float, 16); default: GLA_CASE(float, 32); }
   } else if (dtype == QE_DTYPE_BF16) {

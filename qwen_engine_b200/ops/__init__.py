@@ -1758,7 +1758,7 @@ def linear_attention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, alp
     _check(lib().qe_linear_attention_scan(
         _ptr(q), _ptr(k), _ptr(v), ctypes.c_long(q.stride(0)), ctypes.c_long(k.stride(0)), ctypes.c_long(v.stride(0)),
         _ptr(alpha), _ptr(state), _ptr(ctx.cu_q), _ptr(ctx.ctx_lens), _ptr(ctx.slot_ids), _ptr(out), ctypes.c_float(q_scale),
-        int(ctx.num_reqs), int(ctx.max_q_len), H, dk, dv, int(bool(write_state)), _dt(q), _ptr(da),
+        int(ctx.num_reqs), int(ctx.max_q_len), T, H, dk, dv, int(bool(write_state)), _dt(q), _ptr(da),
         ctypes.c_long(da.stride(0) if da is not None else 0), _ptr(dw), _ptr(db), ctypes.c_float(tau), int(rank),
         _ptr(head_decay), _stream()),
         "linear_attention_scan")

@@ -432,13 +432,19 @@ def test_the_command_line_replays_a_trace(folders, tmp_path):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("H,dk,dv", [(2, 32, 16), (8, 64, 128), (1, 64, 40), (3, 128, 128), (2, 256, 24), (1, 512, 8), (1, 1024, 8), (2, 16, 32)])
-@pytest.mark.parametrize("lens", [[2], [31, 1, 33], [32, 64, 9], [200, 1, 7, 96]])
+@pytest.mark.parametrize("H,dk,dv", [(2, 32, 16), (8, 64, 128), (1, 64, 40), (3, 128, 128), (2, 256, 24), (1, 512, 8), (1, 1024, 8), (2, 16, 32),
+                                     (16, 32, 64), (32, 16, 32)])
+@pytest.mark.parametrize("lens", [[2], [31, 1, 33], [32, 64, 9], [200, 1, 7, 96], [170, 150, 161, 163]])
 @pytest.mark.parametrize("constant", [False, True])
 def test_scan_of_whole_pieces_gives_the_general_paths_bits(ops, dtype, H, dk, dv, lens, constant):
     """Rows in whole pieces of 16 bytes go through a ring of asynchronous copies (chunks of 8 to 32 tokens, their edges, tails of a turn of
     eight, requests of one token among others, columns behind the last): the same bits, outputs and states, as rows that
-    start an element off, which the general kernel stages itself; a decay per channel, or one per head."""
+    start an element off, which the general kernel stages itself; a decay per channel, or one per head.  (Those that stay with the
+    general kernel compare its own two ways of staging.)"""
+    pieces = not (dtype == torch.bfloat16 and (dk == 16 or dk == 1024))          # 4 channels a thread; 4 value channels a CTA
+    pays = max(lens) <= 128 or dk >= 256 or (max(lens) == 170 and H * dv >= 384) or (max(lens) == 200 and H * dv >= 1024)
+    streams = ops.lib().qe_linear_attention_scan_streams(len(lens), max(lens), sum(lens), H, dk, dv, ops._DT[dtype])
+    assert bool(streams) == (pieces and pays)
     T, width = sum(lens), 2 * H * dk + H * dv
     g = torch.Generator().manual_seed(dk + dv + T)
     rows = torch.randn(T, width, generator=g).to(dtype).to(DEV)

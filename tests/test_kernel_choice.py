@@ -90,3 +90,25 @@ def test_few_rows_share_k_where_the_streaming_kernel_takes_a_second_round_or_two
             for K in (512, 1024, 1536, 2048, 4096, 9728):
                 s = got(M, N, K)
                 assert s == 0 or (-(-N // 128) * s <= ops.SPLITK_MAX_CTAS and -(-K // 64) >= 2 * s)
+
+
+def test_the_scan_of_a_long_prompt_stays_with_the_kernel_that_stages_ahead():
+    """... alone and beside requests of few tokens, whatever their number of CTAs; prompts of like lengths, short ones, 256 key channels
+    and more go through the ring of asynchronous copies."""
+    def ring(lens, H=8, dk=64, dv=128, dtype=1):
+        return bool(ops.lib().qe_linear_attention_scan_streams(len(lens), max(lens), sum(lens), H, dk, dv, dtype))
+    assert ops._DT[BF] == 1 and ops._DT[torch.float32] == 0
+    for dtype in (0, 1):
+        for alone in ([2048], [512], [130]):
+            assert not ring(alone, dtype=dtype)
+        for beside in ([512] + [1] * 3, [2048] + [1] * 3, [2048] + [1] * 15, [1024, 64], [1000] + [30] * 8):
+            assert not ring(beside, dtype=dtype)
+        assert not ring([2048] + [1] * 3, H=16, dtype=dtype) and not ring([2048] + [1] * 15, H=16, dtype=dtype)
+        assert not ring([2048] + [1] * 15, H=4, dk=128, dtype=dtype) and not ring([512] + [1] * 3, H=8, dk=128, dv=256, dtype=dtype)
+        for many in ([256] * 8, [512, 512], [700, 500, 300], [1024, 200, 100], [512] + [1] * 63, [64] * 32, [9], [100], [128], [1, 2]):
+            assert ring(many, dtype=dtype)
+        assert ring([2048], H=2, dk=256, dv=64, dtype=dtype) and ring([512] + [1] * 15, H=1, dk=512, dv=64, dtype=dtype)
+        assert not ring([1]) and not ring([1] * 64), "single tokens have a form of their own"
+    assert ring([512] + [1] * 15, H=8, dk=128, dv=256) and not ring([512] + [1] * 15, H=8, dk=128, dv=256, dtype=0)
+    assert not ring([9], dk=16, dtype=1) and ring([9], dk=16, dtype=0), "a thread's channels are not whole pieces"
+    assert not ring([9], dk=72) and not ring([9], dv=132)
