@@ -1378,8 +1378,8 @@ def few_token_parts(geo, keys: list[int], rows: int):
     far as they fit.
 
     The longest part sets the time: 0.0091 us a key.  Parts that meet in a cluster cost next to nothing; parts that are added up through memory
-    as much as 300 keys and 15 for each row, whichever requests they belong to.  So contexts of about equal lengths form
-    clusters, others get parts by their lengths, and where neither shortens the longest by more than that they stay whole, or
+    as much as 350 keys and 15 for each row, whichever requests they belong to.  So contexts of about equal lengths, none of
+    them of less than 32 keys a part, form clusters, others get parts by their lengths, and where neither shortens the longest by more than that they stay whole, or
     go to CTAs of 4 warps, two per SM, by ``parts_for_lengths``'s rule.  From five rows on 8 parts of less than a split each are
     1.1 to 1.3 times as slow as 4 (16 / 8 heads, 4 tokens behind 600 and 1 700 keys 8.5, 9.8 us / 6.4, 8.1; 2 tokens 4.5, 5.7 / 4.8, 6.5), and 36 clusters of 4
     do not all find room (16 / 2 heads, 18 requests of 1 300 keys 28.0 us, in clusters of 2 14.4).
@@ -1401,8 +1401,8 @@ def few_token_parts(geo, keys: list[int], rows: int):
     slots = TC_TARGET_CTAS // base
     dealt = parts_by_length(keys, slots) if DECODE_PARTS_BY_LENGTH and n < slots else None
     longest = max(-(-k // p) for k, p in zip(keys, dealt)) if dealt else span
-    cost = 300 + 15 * rows
-    if parts in (2, 4, 8) and -(-span // parts) <= longest + cost:
+    cost = 350 + 15 * rows
+    if parts in (2, 4, 8) and min(keys) >= 32 * parts and -(-span // parts) <= longest + cost:
         return parts
     if longest + cost <= span:
         total = TotalParts(sum(dealt))
