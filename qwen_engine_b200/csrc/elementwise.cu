@@ -458,28 +458,33 @@ __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ q, T* __restrict__ 
   }
 }
 
-// U neighbouring heads of a token per warp, all of q, all of k or all of v, their loads in flight together (large steps: U = 4;
-// the launcher's rule): one set of angles, norm weights and one cache slot serve them.  Position, weights and slot, and the
+// U neighbouring heads of a token per warp, their loads in flight together (large steps: U = 4; the launcher's rule): one set
+// of angles, norm weights and one cache slot serve them.  All of q, all of k or all of v; MIXED: of any kind, the token's
+// last warp with what is left over.  Position, weights and slot, and the
 // angles where the step has no table of them, are fetched and worked out while the kernel before this one (the QKV
 // product) is still running; a table's angles together with the elements.  Measured on a B200, a chain of launches, against
 // four heads of any kind with their angles, weights and slots behind the norm's sum: 527 tokens of 16 / 8 heads 5.8 -> 4.7 us, 141
 // 4.0 -> 3.1; float32, against the general kernel's loop over the head, 9.7 -> 3.9 and 4.7 -> 3.1, one token 3.1 -> 1.4.
-template <typename T, int U>
+// MIXED, the same, and one head a warp in brackets: 2 048 tokens of 16 / 2 heads 9.7 -> 8.9 (11.4), 8 192 31.7 -> 30.3 (41.7), of 12 / 2 25.9 ->
+// 24.3 (33.5), of 5 / 1 13.0 -> 12.1 (15.4), of 7 / 7 34.0 -> 33.4 (41.7), of 15 / 5 39.9 -> 40.3 (50.8); float32 8 192 of 16 / 2 82 -> 41 (63).
+template <typename T, int U, bool MIXED>
 __global__ void qk_norm_rope_kv_write_d128_kernel(RopeD128Args<T> args) {
   pdl_launch_dependents();
   // the launcher keeps tokens x heads below 2^31
   const int heads_total = args.Hq + 2 * args.Hkv;
-  const int item = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * U;
-  const int t = item / heads_total, head = item - t * heads_total;
+  const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int groups = MIXED ? (heads_total + U - 1) / U : heads_total / U;      // of a token
+  const int t = warp / groups, head = (warp - t * groups) * U;
+  const int n = MIXED ? min(U, heads_total - head) : U;
   RopeD128Pre pre;
-  rope_d128_prepare(args, t, head, pre);
+  rope_d128_prepare<MIXED>(args, t, head, head + n - 1, pre);
   pdl_wait();
   RopeRaw<T> raw[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) raw[u] = rope_d128_load(args, t, head + u);
+  for (int u = 0; u < U; ++u) if (u < n) raw[u] = rope_d128_load(args, t, head + u);
   rope_d128_angles(args, t, head, pre);
 #pragma unroll
-  for (int u = 0; u < U; ++u) rope_d128_finish(args, t, head + u, raw[u], pre);
+  for (int u = 0; u < U; ++u) if (u < n) rope_d128_finish<MIXED>(args, t, head + u, raw[u], pre);
 }
 
 // cos_sin[t, j] = (cos, sin)(positions[t] * inv_freq[j]) in float32: the angles of a step, computed
@@ -520,10 +525,16 @@ static int launch_rope_d128(void* q, void* k, const void* v, long q_stride, long
   const int vwarps = 8;
   const RopeD128Args<T> ra{(T*)q, (T*)k, (const T*)v, q_stride, k_stride, v_stride, positions, qw, kw, eps, inv_freq, (const float2*)cos_sin,
                            (T*)pages, slot_mapping, tokens, Hq, Hkv, page_size, write_kv};
+  const int heads = Hq + 2 * Hkv;
+  auto grid = [&](long warps) { return dim3((unsigned)((warps + vwarps - 1) / vwarps)); };
+  // Four heads a warp need many of them to fill the SMs; where they are not of one kind, and some places stay empty, the line is
+  // higher (16 / 2 heads, one / four: 600 tokens 4.0 / 4.7 us, 1 000 5.9 / 4.8; 5 / 1, 2 048 4.6 / 4.5; 7 / 7, 1 000 5.9 / 6.4, 2 048 11.4 / 10.8).
   if (n_items >= 4096 && Hq % 4 == 0 && Hkv % 4 == 0)
-    qe_launch(qk_norm_rope_kv_write_d128_kernel<T, 4>, dim3((unsigned)((n_items + 4 * vwarps - 1) / (4 * vwarps))), dim3(vwarps * 32), 0, stream, ra);
+    qe_launch(qk_norm_rope_kv_write_d128_kernel<T, 4, false>, grid(n_items / 4), dim3(vwarps * 32), 0, stream, ra);
+  else if (n_items >= 16384)
+    qe_launch(qk_norm_rope_kv_write_d128_kernel<T, 4, true>, grid((long)tokens * ((heads + 3) / 4)), dim3(vwarps * 32), 0, stream, ra);
   else
-    qe_launch(qk_norm_rope_kv_write_d128_kernel<T, 1>, dim3((unsigned)((n_items + vwarps - 1) / vwarps)), dim3(vwarps * 32), 0, stream, ra);
+    qe_launch(qk_norm_rope_kv_write_d128_kernel<T, 1, false>, grid(n_items), dim3(vwarps * 32), 0, stream, ra);
   QE_CHECK_LAUNCH("qk_norm_rope_kv_write");
   return 0;
 }

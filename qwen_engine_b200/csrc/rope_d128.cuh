@@ -65,21 +65,24 @@ __device__ __forceinline__ RopeRaw<T> rope_d128_load(const RopeD128Args<T>& A, i
 // its predecessor.  Angles only where the step has no table of them.
 struct RopeD128Pre {
   float cs[4], sn[4];
-  float4 wv;
+  float4 wv;                        // the norm's weights: those of the first head's kind
+  float4 wk;                        // MIXED: k's, for a warp that has heads of q and of k
   int slot;
 };
-template <typename T>
-__device__ __forceinline__ void rope_d128_prepare(const RopeD128Args<T>& A, int t, int head, RopeD128Pre& P) {
+// (for heads `head` to `last` of token t; MIXED: they may be of several kinds, q, k and v)
+template <bool MIXED, typename T>
+__device__ __forceinline__ void rope_d128_prepare(const RopeD128Args<T>& A, int t, int head, int last, RopeD128Pre& P) {
   const int lane = threadIdx.x & 31;
   P.slot = 0;
   P.wv = make_float4(1.f, 1.f, 1.f, 1.f);
 #pragma unroll
   for (int i = 0; i < 4; ++i) { P.cs[i] = 1.f; P.sn[i] = 0.f; }
   if (t >= A.T_tokens) return;
-  if (A.write_kv && head >= A.Hq) P.slot = __ldg(A.slot_mapping + t);
+  if (A.write_kv && last >= A.Hq) P.slot = __ldg(A.slot_mapping + t);
   if (head >= A.Hq + A.Hkv) return;
   const float* w = head < A.Hq ? A.qw : A.kw;
   if (w) P.wv = __ldg(reinterpret_cast<const float4*>(w + 4 * lane));
+  if (MIXED) P.wk = A.kw && last >= A.Hq ? __ldg(reinterpret_cast<const float4*>(A.kw + 4 * lane)) : P.wv;
   if (A.inv_freq && !A.cos_sin) {
     const float pos = (float)__ldg(A.positions + t);
 #pragma unroll
@@ -99,7 +102,7 @@ __device__ __forceinline__ void rope_d128_angles(const RopeD128Args<T>& A, int t
   P.cs[2] = t23.x; P.sn[2] = t23.y; P.cs[3] = t23.z; P.sn[3] = t23.w;
 }
 
-template <typename T>
+template <bool MIXED, typename T>
 __device__ __forceinline__ void rope_d128_finish(const RopeD128Args<T>& A, int t, int head, const RopeRaw<T>& raw,
                                                  const RopeD128Pre& pre) {
   constexpr int D = 128;
@@ -128,7 +131,7 @@ __device__ __forceinline__ void rope_d128_finish(const RopeD128Args<T>& A, int t
   if (w) {
     const float ss = warp_sum(f[0] * f[0] + f[1] * f[1] + f[2] * f[2] + f[3] * f[3]);
     const float rstd = rsqrtf(ss / (float)D + eps);
-    const float4 wv = pre.wv;
+    const float4 wv = MIXED && !is_q ? pre.wk : pre.wv;
     f[0] = f[0] * rstd * wv.x; f[1] = f[1] * rstd * wv.y; f[2] = f[2] * rstd * wv.z; f[3] = f[3] * rstd * wv.w;
   }
   if (A.inv_freq) {

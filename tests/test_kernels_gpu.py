@@ -457,6 +457,44 @@ def test_qk_norm_rope_kv_write(dtype, Hq, Hkv, D, P, rot, norm):
     assert float(flat[mask].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T,Hq,Hkv,P", [(127, 16, 8, 16), (128, 16, 8, 16), (131, 16, 8, 3), (1023, 12, 2, 16), (1024, 12, 2, 16), (911, 14, 2, 5),
+                                        (2345, 5, 1, 16), (781, 7, 7, 16), (656, 15, 5, 4), (5500, 1, 1, 16)])
+@pytest.mark.parametrize("table", [True, False])
+@pytest.mark.parametrize("norm,write_kv", [(True, True), (False, True), (True, False)])
+def test_qk_norm_rope_kv_write_of_many_tokens(dtype, T, Hq, Hkv, P, table, norm, write_kv):
+    """Head size 128, 4 096 (token, head) pairs and more: a warp takes four neighbouring heads of a token, from 16 384 on also
+    where they are of several kinds and the last warp of a token has fewer (and pairs just below the lines: one a warp),
+    with the step's table of angles and without; rows that are the leading columns of a wider product."""
+    D = 128
+    W = (Hq + 2 * Hkv) * D
+    qkv = _randn((T, W + 8), dtype, 91)[:, :W]
+    g = torch.Generator().manual_seed(92)
+    positions = torch.randint(0, 40000, (T,), generator=g, dtype=torch.int32)
+    qw = (1 + 0.2 * _randn((D,), torch.float32, 93)) if norm else None
+    kw = (1 + 0.2 * _randn((D,), torch.float32, 94)) if norm else None
+    inv_freq = 1.0 / (1e6 ** (torch.arange(0, D, 2, dtype=torch.float32) / D))
+    pages = -(-T // P) + 2
+    slots = torch.randperm(pages * P, generator=g)[:T].to(torch.int32)
+    cache_ref, qkv_ref = torch.zeros(pages, 2, Hkv, P, D, dtype=dtype), qkv.clone()
+    ref_ops.qk_norm_rope_kv_write(qkv_ref, positions, qw, kw, 1e-6, inv_freq, D, cache_ref, slots, Hq, Hkv, D, write_kv=write_kv)
+    cache, wide = torch.zeros(pages, 2, Hkv, P, D, dtype=dtype, device=DEV), torch.zeros(T, W + 8, dtype=dtype, device=DEV)
+    got = wide[:, :W]
+    got.copy_(qkv)
+    angles = None
+    if table:
+        angles = torch.empty(T, D // 2, 2, device=DEV)
+        ops.rope_table(positions.to(DEV), inv_freq.to(DEV), angles)
+    ops.qk_norm_rope_kv_write(got, positions.to(DEV), qw.to(DEV) if norm else None, kw.to(DEV) if norm else None, 1e-6, inv_freq.to(DEV), D,
+                              cache, slots.to(DEV), Hq, Hkv, D, write_kv=write_kv, cos_sin=angles)
+    _close(got, qkv_ref, dtype, tol32=3e-5)
+    _close(cache, cache_ref, dtype, tol32=3e-5)
+    written = torch.zeros(pages * P, dtype=torch.bool)
+    written[slots.long()] = write_kv
+    assert float(cache.cpu().permute(0, 3, 1, 2, 4).reshape(pages * P, -1)[~written].abs().max()) == 0.0
+    assert float(wide[:, W:].abs().max()) == 0.0 and torch.equal(got[:, (Hq + Hkv) * D:].cpu(), qkv[:, (Hq + Hkv) * D:])
+
+
 @pytest.mark.parametrize("T,Hq,Hkv,K,P", [(300, 4, 2, 136, 16), (1000, 3, 1, 72, 4), (2048, 16, 8, 1024, 16), (257, 2, 2, 64, 256)])
 @pytest.mark.parametrize("norm", [True, False])
 @pytest.mark.parametrize("write_kv", [True, False])
