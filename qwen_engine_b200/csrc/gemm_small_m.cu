@@ -13,9 +13,10 @@
 // fixed order.  Any N; K a multiple of 8 (16-byte rows); the launcher refuses the rest.
 #include "gemm_small_m.cuh"
 
-// PER_SM: CTAs of 8 warps that an SM has registers for (0: up to 16 warps, one CTA or more).
-template <int MT, typename TOut, int XMODE, bool RESID, int ROWS = 16, int PER_SM = 0>
-__global__ void __launch_bounds__(PER_SM ? 256 : 512, PER_SM)
+// WARPS: the most warps of a CTA.  With 8 the compiler keeps to 74 registers a thread (one tile of tokens), with 16 to 82; asked for
+// three CTAs an SM, which 74 allow, it spilled 24 to 36 bytes a thread.
+template <int MT, typename TOut, int XMODE, bool RESID, int ROWS = 16, int WARPS = 16>
+__global__ void __launch_bounds__(WARPS * 32)
 gemm_small_m_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                     TOut* __restrict__ out, int M, int N, int K, int k_per_warp, FuseArgs na) {
   extern __shared__ float red[];                    // [warps][16][8 MT]
@@ -210,14 +211,14 @@ static int launch_small_m(const void* x, const void* w, void* out, int M, int N,
   }
   if constexpr (MT == 1 && XMODE == X_PLAIN && !RESID) {
     // More CTAs than two per SM: with 82 registers a thread only two of 8 warps fit, and what was left over waited for
-    // a second round (6 144 x 2 560, 384 CTAs, at 1 and 8 rows 10.4 and 11.4 us, with 80 registers 7.8 and 8.1; 5 120 x 1 024
-    // 4.9 and 5.2, now 2.8 and 3.0).
+    // a second round (6 144 x 2 560, 384 CTAs, at 1 and 8 rows 10.4 and 11.4 us, with 74 registers 7.4 and 8.2; 5 120 x 1 024
+    // 4.9 and 5.2, now 2.7 and 3.0).
     if (ctas > 2 * 148 && warps <= 8) {
       if (out_f32)
-        qe_launch(gemm_small_m_kernel<MT, float, XMODE, RESID, 16, 3>, dim3(ctas), dim3(warps * 32), smem, stream,
+        qe_launch(gemm_small_m_kernel<MT, float, XMODE, RESID, 16, 8>, dim3(ctas), dim3(warps * 32), smem, stream,
                   (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (float*)out, M, N, K, k_per_warp, na);
       else
-        qe_launch(gemm_small_m_kernel<MT, __nv_bfloat16, XMODE, RESID, 16, 3>, dim3(ctas), dim3(warps * 32), smem, stream,
+        qe_launch(gemm_small_m_kernel<MT, __nv_bfloat16, XMODE, RESID, 16, 8>, dim3(ctas), dim3(warps * 32), smem, stream,
                   (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, M, N, K, k_per_warp, na);
       QE_CHECK_LAUNCH("linear_small_m");
       return 0;
@@ -243,6 +244,18 @@ extern "C" int qe_small_m_prefetch_next(const void* w, unsigned long long bytes)
   g_next_w = (const unsigned char*)w;
   g_next_bytes = w ? bytes : 0;
   return 0;
+}
+
+// How many CTAs of 8 warps of the form for many weight rows (see launch_small_m) an SM takes, and the bytes of local memory of
+// a thread (a test asks: three, and none).
+extern "C" int qe_small_m_ctas_per_sm(int out_f32, int* local_bytes) {
+  const void* kernel = out_f32 ? (const void*)gemm_small_m_kernel<1, float, X_PLAIN, false, 16, 8> : (const void*)gemm_small_m_kernel<1, __nv_bfloat16, X_PLAIN, false, 16, 8>;
+  cudaFuncAttributes attr;
+  int ctas = 0;
+  if (cudaFuncGetAttributes(&attr, kernel) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kernel, 256, 8 * 16 * 8 * sizeof(float)) != cudaSuccess) return -1;
+  if (local_bytes) *local_bytes = (int)attr.localSizeBytes;
+  return ctas;
 }
 
 template <int XMODE, bool RESID>

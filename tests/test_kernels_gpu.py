@@ -1257,6 +1257,13 @@ def test_linear_of_few_rows_against_more_than_a_round_of_weights(M, N, K, out_f3
         _close(got, want, odt, tol16=8e-3)
 
 
+@pytest.mark.parametrize("out_f32", [0, 1])
+def test_three_ctas_of_a_product_against_many_weight_rows_fit_an_sm(out_f32):
+    import ctypes
+    local = ctypes.c_int(-1)
+    assert ops.lib().qe_small_m_ctas_per_sm(out_f32, ctypes.byref(local)) >= 3 and local.value == 0
+
+
 @pytest.mark.parametrize("Hq,Hkv,D,P", [(16, 8, 128, 16), (4, 2, 64, 8), (6, 2, 256, 16), (6, 2, 48, 4)])
 @pytest.mark.parametrize("n,ctx", [(9, 300), (20, 700), (31, 2100), (23, 9000)])
 @pytest.mark.parametrize("sinks", [False, True])
