@@ -56,6 +56,9 @@ __device__ __forceinline__ void dm_ldsm_x4_t(uint32_t (&r)[4], uint32_t a) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
+// 2^x by the instruction alone, results below 2^-126 as zero (exp2f keeps them as subnormals, at 0.5 to 2 % of the launch: one request
+// of 1 088 keys 4.78 -> 4.88 us, 8 9.71 -> 9.76, 28 24.98 -> 25.25).  A warp's largest weight is 1, so what is lost is less than
+// 2^-126 of the sum of its weights, and a key's less than 2^-126 of its value.
 __device__ __forceinline__ float dm_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
@@ -344,7 +347,7 @@ decode_attention_mma_kernel(FaArgs A_launch, long long prefetch_delta, int early
     cp_async_wait<DM_STAGES - 1>();                 // all but the latest commits of the other stages have landed: this group has
     __syncwarp();
     const int j0 = kv_begin + gidx * DM_GK;
-    const bool all_allowed = j0 >= kv_begin && j0 + DM_GK <= kv_end && j0 + DM_GK - 1 <= first_pos && (window <= 0 || j0 > last_pos - window);
+    const bool all_allowed = j0 + DM_GK <= kv_end && j0 + DM_GK - 1 <= first_pos && (window <= 0 || j0 > last_pos - window);
     const uint32_t tk = stage0 + (uint32_t)st * (2 * DM_TILE_BYTES);
     dm_tile<HI>(q, tk + k_lane, tk + DM_TILE_BYTES + v_lane, j0, kv_begin, kv_end, pos_lo, pos_hi, window, A.scale_log2, cap_in, cap_out,
                 biased, slope_lo, slope_hi, all_allowed, lane, m_lo, m_hi, l_lo, l_hi, o);

@@ -1318,6 +1318,21 @@ def test_a_few_tokens_of_every_request_in_parts_by_length(Hq, Hkv, q_lens, ctx_l
     _close(got, want, dtype)
 
 
+@pytest.mark.parametrize("Hq,Hkv,q_lens", [(8, 1, [1, 1, 1, 1]), (9, 1, [1, 1, 1, 1]), (4, 1, [2, 1, 1, 2]), (4, 1, [3, 1, 2, 1]), (16, 1, [1, 1, 1, 1])])
+@pytest.mark.parametrize("window", [0, 50])
+@pytest.mark.parametrize("options", [{}, {"sinks": True}, {"softcap": 20.0}, {"slopes": True}, {"softcap": 5.0, "sinks": True}])
+def test_decode_attention_of_eight_rows_and_more(Hq, Hkv, q_lens, window, options):
+    """8 rows an item (the upper half of the instruction's rows is left out) and 9 to 16, with everything that bends, biases or masks a score,
+    at contexts that end within a group of 16 keys, at one's end and behind it."""
+    P, dtype, ctx_lens = 16, torch.bfloat16, [14, 15, 16, 333]
+    options = {k: torch.linspace(0.01, 0.6, Hq) if v is True else v for k, v in options.items()}
+    case = _attention_case(dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, window, seed=89)
+    want = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, window, ref_ops.paged_attention, "cpu", **options)
+    got = _run_attention(case, dtype, Hq, Hkv, 128, P, q_lens, ctx_lens, window, ops.paged_attention, DEV, **options)
+    assert ops.last_attention_kernel == "decode_attention_mma"
+    _close(got, want, dtype)
+
+
 @pytest.mark.parametrize("T", [1, 3, 40])
 @pytest.mark.parametrize("H", [256, 512, 768, 1024, 1280, 1536, 1792, 2048, 2560, 3072, 3584, 4096])
 @pytest.mark.parametrize("with_delta", [False, True])
