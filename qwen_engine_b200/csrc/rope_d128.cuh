@@ -91,7 +91,8 @@ __device__ __forceinline__ void rope_d128_prepare(const RopeD128Args<T>& A, int 
 }
 
 // The angles from the step's table, where it has one: a kernel of the step made it, so they are asked for after the wait, but
-// together with the elements (behind the norm's sum they were a second round trip).
+// together with the elements (behind the norm's sum they were a second round trip).  The models make a table for
+// bfloat16 alone; the entry point takes one for either type.
 template <typename T>
 __device__ __forceinline__ void rope_d128_angles(const RopeD128Args<T>& A, int t, int head, RopeD128Pre& P) {
   if (!A.inv_freq || !A.cos_sin || t >= A.T_tokens || head >= A.Hq + A.Hkv) return;

@@ -512,9 +512,10 @@ def few_rows_splits(M: int, N: int, K: int, dtype: torch.dtype) -> int:
     second round, and from 9 rows on an instruction covers two tiles of tokens.  Measured on a B200 (a chain of launches over
     weights beyond L2; streaming / clusters), 9 and 16 rows: in clusters of 4 2 432 x 1 536 4.6, 5.0 / 4.3, 4 096 x 2 048 6.3,
     6.8 / 5.6, 4 096 x 4 096 10.8, 12.0 / 8.3, but x 1 024 3.8, 4.1 / 4.3, and 4 736 x 2 048 6.4 / 9.2 (74 clusters of 4 do not all
-    find room); in clusters of 2 6 144 x 2 560 9.3, 9.8 / 7.9, but 5 120 x 2 048 6.5, 7.2 / 7.1; more than three CTAs per SM,
-    7 168 x 1 024 7.3, 7.8 / 5.1, 8 192 x 2 560 16.2, 17.7 / 9.0.  At 1 and 8 rows 8 192 x 1 536 8.4, 8.9 / 6.4, 6 144 x 4 096 11.8,
-    13.3 / 10.9, but 9 216 x 1 024 5.4 / 6.0 and 5 120 x 4 096 9.3, 9.9 / 10.1."""
+    find room); in clusters of 2 6 144 x 2 560 9.3, 9.8 / 7.9, 4 224 to 5 120 x 2 560 8.3-8.5, 8.9-9.2 / 6.7-7.8, but 5 120 x 2 048 6.5,
+    7.2 / 7.1; more than three CTAs per SM, 7 168 x 1 024 7.3, 7.8 / 5.1, 8 192 x 2 560 16.2, 17.7 / 9.0.  At 1 and 8 rows 8 192 x 1 536 7.4,
+    8.1 / 6.4, 6.7, 6 144 x 6 144 14.9, 15.5 / 14.7, 14.8 (x 4 096 10.3, 10.7 / 10.8, 10.9: about even), but 9 216 x 1 024 5.2, 6.1 / 6.1, 6.0 and
+    5 120 x 4 096 8.9, 9.3 / 10.2."""
     if not (TCGEN05_ENABLED and SPLITK and dtype == torch.bfloat16 and 1 <= M <= 16 and K % 8 == 0 and N % 4 == 0):
         return 0
     ctas, tiles = -(-N // 16), -(-N // 128)
